@@ -11,6 +11,8 @@
 // chains of length ~n; k_color_chunked below bounds the work by walking
 // index-ordered chunks instead.
 
+#include <algorithm>
+
 #include "color.cuh"
 
 namespace cc {
@@ -21,11 +23,13 @@ __device__ __forceinline__ void mark(unsigned long long& mask, uint32_t c, bool&
 }
 
 // Greedy rule for one vertex: smallest colour not used by a lower-index
-// neighbour (material graph, contact co-vertices, grab).
-__device__ __forceinline__ uint32_t greedy_color(const ColorView& g, const uint16_t* cin, uint32_t v) {
+// neighbour (material graph, contact co-vertices, grab). color_of(u) gives a
+// neighbour's current colour.
+template <class ColorOf>
+__device__ __forceinline__ uint32_t greedy_color(const ColorView& g, uint32_t v, ColorOf color_of) {
     unsigned long long mask = 0;
     bool high = false;
-    for (uint32_t k = g.lo_off[v]; k < g.lo_off[v + 1]; ++k) mark(mask, cin[g.lo[k]], high);
+    for (uint32_t k = g.lo_off[v]; k < g.lo_off[v + 1]; ++k) mark(mask, color_of(g.lo[k]), high);
     for (uint32_t k = g.contacts.inc_off[v]; k < g.contacts.inc_off[v + 1]; ++k) {
         uint32_t c = g.contacts.inc[k];
         uint32_t kind = g.contacts.kind[c];
@@ -33,155 +37,416 @@ __device__ __forceinline__ uint32_t greedy_color(const ColorView& g, const uint1
         uint32_t ids[4] = {cv.x, cv.y, cv.z, cv.w};
         uint32_t cnt = kind == 0 ? 2u : (kind == 1 ? 3u : 4u);
         for (uint32_t j = 0; j < cnt; ++j)
-            if (ids[j] < v) mark(mask, cin[ids[j]], high);
+            if (ids[j] < v) mark(mask, color_of(ids[j]), high);
     }
     bool in_grab = g.grab_active && (g.grab_v[0] == v || g.grab_v[1] == v || g.grab_v[2] == v);
     if (in_grab)
         for (int j = 0; j < 3; ++j)
-            if (g.grab_v[j] < v) mark(mask, cin[g.grab_v[j]], high);
+            if (g.grab_v[j] < v) mark(mask, color_of(g.grab_v[j]), high);
     if (~mask != 0ull) return (uint32_t)__ffsll((long long)~mask) - 1;
     for (uint32_t col = 64;; ++col) {  // more than 64 colours around v: linear search
         bool used = false;
-        for (uint32_t k = g.lo_off[v]; k < g.lo_off[v + 1] && !used; ++k) used = cin[g.lo[k]] == col;
+        for (uint32_t k = g.lo_off[v]; k < g.lo_off[v + 1] && !used; ++k) used = color_of(g.lo[k]) == col;
         for (uint32_t k = g.contacts.inc_off[v]; k < g.contacts.inc_off[v + 1] && !used; ++k) {
             uint32_t c = g.contacts.inc[k];
             uint32_t kind = g.contacts.kind[c];
             uint4 cv = g.contacts.verts[c];
             uint32_t ids[4] = {cv.x, cv.y, cv.z, cv.w};
             uint32_t cnt = kind == 0 ? 2u : (kind == 1 ? 3u : 4u);
-            for (uint32_t j = 0; j < cnt; ++j) used = used || (ids[j] < v && cin[ids[j]] == col);
+            for (uint32_t j = 0; j < cnt; ++j) used = used || (ids[j] < v && color_of(ids[j]) == col);
         }
         if (in_grab)
-            for (int j = 0; j < 3; ++j) used = used || (g.grab_v[j] < v && cin[g.grab_v[j]] == col);
+            for (int j = 0; j < 3; ++j) used = used || (g.grab_v[j] < v && color_of(g.grab_v[j]) == col);
         if (!used || col >= kMaxColors - 1) return col;
     }
 }
 
+// Distinct lower neighbours of every vertex, one row per vertex, built by the
+// whole GPU before the walk (k_color_rows), so that the walk's one block reads
+// each neighbour once: in layered cloth a vertex has the same neighbour in
+// many contacts (the 201 x 311 roll: 40 contacts a vertex, ~120 entries, ~20
+// distinct lower neighbours).
+constexpr int kChunk = 1024;       // vertices of one walk step
+constexpr int kRowSlots = 64;      // distinct lower neighbours a row can hold
+constexpr uint32_t kRowSlow = ~0u;  // count word of a vertex that takes the full rule instead
+constexpr int kRowLanes = 8;       // threads per row
+
+struct ColorRows {
+    uint32_t* adj;  // rows: neighbours below the vertex's chunk, then those in it (outside its 32-group)
+    // [n] .x first entry of the row / 4; .y entries below the chunk | in the chunk << 16, or kRowSlow;
+    // .z lower neighbours among the vertex's 32-aligned group, one bit each; .w unused
+    uint4* head;
+};
+// First entry of v's row, 16-byte aligned: a vertex has at most its material
+// neighbours, 3 vertices per contact and 2 of the grab; 3 more are lost to the
+// alignment.
+__host__ __device__ __forceinline__ size_t row_bound(size_t lo, size_t inc, size_t v) { return lo + 3 * inc + 5 * v; }
+__device__ __forceinline__ size_t row_start(const ColorView& g, uint32_t v) {
+    return (row_bound(g.lo_off[v], g.contacts.inc_off[v], v) + 3) & ~(size_t)3;
+}
+
+// Rows, and the lowest vertex whose rule fails for the current colouring
+// (`first`). Eight threads per vertex put its lower neighbours into a 64-slot
+// hash set in shared memory. Bound by the latency of inc -> contact -> colour.
+__global__ void __launch_bounds__(128) k_color_rows(ColorView g, ColorRows r, const uint16_t* col, unsigned int* first) {
+    __shared__ uint32_t slots[128 / kRowLanes][kRowSlots];
+    __shared__ uint32_t group_bits[128 / kRowLanes];
+    constexpr uint32_t kEmpty = ~0u;
+    const uint32_t lane = threadIdx.x & (kRowLanes - 1), row = threadIdx.x / kRowLanes;
+    const unsigned gmask = ((1u << kRowLanes) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(kRowLanes - 1));
+    uint32_t* slot = slots[row];
+    constexpr uint32_t kPer = 128 / kRowLanes;
+    for (uint32_t v = blockIdx.x * kPer + row; v < g.n; v += gridDim.x * kPer) {  // whole groups step together
+        for (int k = lane; k < kRowSlots; k += kRowLanes) slot[k] = kEmpty;
+        if (lane == 0) group_bits[row] = 0u;
+        __syncwarp(gmask);
+        bool full = false;
+        auto insert = [&](uint32_t u) {
+            if (u >= v) return;
+            if ((u >> 5) == (v >> 5)) {
+                atomicOr(&group_bits[row], 1u << (u & 31u));
+                return;
+            }
+            uint32_t h = (u * 2654435761u) >> 26;
+            for (int tries = 0; tries < kRowSlots; ++tries, h = (h + 1) & (kRowSlots - 1)) {
+                const uint32_t old = atomicCAS(&slot[h], kEmpty, u);
+                if (old == kEmpty || old == u) return;
+            }
+            full = true;
+        };
+        for (uint32_t k = g.lo_off[v] + lane; k < g.lo_off[v + 1]; k += kRowLanes) insert(g.lo[k]);
+        for (uint32_t k = g.contacts.inc_off[v] + lane; k < g.contacts.inc_off[v + 1]; k += kRowLanes) {
+            uint32_t c = g.contacts.inc[k];
+            uint32_t kind = g.contacts.kind[c];
+            uint4 cv = g.contacts.verts[c];
+            insert(cv.x);
+            insert(cv.y);
+            if (kind > 0) insert(cv.z);
+            if (kind > 1) insert(cv.w);
+        }
+        if (lane == 0 && g.grab_active && (g.grab_v[0] == v || g.grab_v[1] == v || g.grab_v[2] == v))
+            for (int j = 0; j < 3; ++j) insert(g.grab_v[j]);
+        __syncwarp(gmask);
+        full = __any_sync(gmask, full);
+        const uint32_t bits = group_bits[row];
+        const uint32_t base = v & ~(uint32_t)(kChunk - 1);
+        // this lane's slots: those below the chunk, then those in it
+        uint32_t n_out = 0, n_in = 0;
+        unsigned long long mask = 0;
+        bool high = full;
+        for (int k = lane; k < kRowSlots; k += kRowLanes) {
+            const uint32_t u = slot[k];
+            if (u == kEmpty) continue;
+            if (u < base) ++n_out;
+            else ++n_in;
+            mark(mask, col[u], high);
+        }
+        for (uint32_t b = lane; b < 32; b += kRowLanes)
+            if (bits >> b & 1u) mark(mask, col[(v & ~31u) + b], high);
+        uint32_t o0 = n_out, i0 = n_in;  // inclusive prefix over the group's lanes
+        for (int o = 1; o < kRowLanes; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(gmask, o0, o, kRowLanes), c = __shfl_up_sync(gmask, i0, o, kRowLanes);
+            if ((int)lane >= o) {
+                o0 += a;
+                i0 += c;
+            }
+        }
+        const uint32_t outs = __shfl_sync(gmask, o0, kRowLanes - 1, kRowLanes);
+        const uint32_t ins = __shfl_sync(gmask, i0, kRowLanes - 1, kRowLanes);
+        o0 -= n_out;
+        i0 -= n_in;
+        if (!full) {
+            uint32_t* out = r.adj + row_start(g, v);
+            for (int k = lane; k < kRowSlots; k += kRowLanes) {
+                const uint32_t u = slot[k];
+                if (u == kEmpty) continue;
+                if (u < base) out[o0++] = u;
+                else out[outs + i0++] = u;
+            }
+        }
+        for (int o = kRowLanes / 2; o > 0; o >>= 1) mask |= __shfl_xor_sync(gmask, mask, o, kRowLanes);
+        high = __any_sync(gmask, high);
+        if (lane == 0) {
+            r.head[v] = make_uint4((uint32_t)(row_start(g, v) / 4), full ? kRowSlow : (outs | ins << 16), bits, 0u);
+            const uint32_t c = (high || ~mask == 0ull) ? greedy_color(g, v, [&](uint32_t u) { return (uint32_t)col[u]; })
+                                                       : (uint32_t)__ffsll((long long)~mask) - 1;
+            if (c != col[v]) atomicMin(first, v);
+        }
+        __syncwarp(gmask);  // the slots are reused
+    }
+}
+
 // Exact sequential-greedy colouring by one CTA: chunks of kChunk consecutive
-// vertices are visited in index order, so every lower neighbour outside the
-// current chunk is already final; inside the chunk the greedy rule is
-// iterated Jacobi-style (read all, barrier, write changes) until no colour
-// changes. A chunk converges in at most (its internal descending chain + 1)
-// rounds <= kChunk + 1, so the loop is bounded; starting from the previous
-// colouring a chunk usually settles in a few rounds.
-//
-// Per chunk each thread first folds the colours of its vertex's final lower
-// neighbours (index below the chunk) into a 64-bit mask, and keeps the
-// in-chunk lower neighbours (at most kInner, as chunk-local indices) in
-// shared memory; the rounds then read only shared memory: the mask, those
-// indices and the chunk's current colours. A vertex with more in-chunk lower
-// neighbours, or with a colour >= 64 around it, takes the full rule
-// (greedy_color) every round instead. Both give the rule's exact value.
+// vertices are visited in index order, so every lower neighbour below the
+// current chunk is already final; inside the chunk the greedy rule is iterated
+// (rounds of one barrier, the chunk's colours double-buffered) until no colour
+// changes. Each thread has one vertex. Once per chunk it folds the colours of
+// its row's neighbours below the chunk into a 64-bit mask; a round adds the
+// in-chunk neighbours of other warps from the last round's colours, and then
+// each warp settles its own 32 vertices exactly (settle_chain, settle). A change
+// therefore crosses a whole warp per round, and after round r the chunk's first
+// r warps are final, so 32 rounds and one that finds no change bound the loop.
+// From the second round on a warp whose neighbour warps did not change in the
+// last one skips the evaluation: a round of all 32 warps is bound by instruction
+// issue, one of a few by their latency alone. A vertex without a row, or with a
+// colour >= 64 around it, takes the full rule (greedy_color) once a round
+// instead; its chunk then needs at most kChunk + 1 rounds.
 //
 // The walk starts at the chunk of `first[0]`, the lowest vertex whose rule
-// does not hold for the previous colouring (k_color_probe): every vertex
+// does not hold for the previous colouring (k_color_rows): every vertex
 // below it already satisfies the rule against final lower neighbours, so it
 // is final too. When the whole colouring fits (n <= kSmemColors) it is kept
 // in shared memory for the walk.
-constexpr int kChunk = 1024;
-constexpr int kInner = 16;
-constexpr uint32_t kSmemColors = 90 * 1024;  // 180 KB of uint16 colours (+ 34 KB static)
-__global__ void __launch_bounds__(kChunk) k_color_chunked(ColorView g, uint16_t* col_g, const unsigned int* first,
-                                                         unsigned int* rounds_out, unsigned int* err) {
-    extern __shared__ uint16_t col_s[];
-    __shared__ uint16_t inner[kInner][kChunk];  // chunk-local indices of in-chunk lower neighbours
-    __shared__ uint16_t chunk_col[kChunk];      // the chunk's current colours
-    uint32_t start = *first;
+//
+// What bounds it: the chain of chunks, each a row load, a gather of final
+// colours and two to three barrier rounds; the next chunk's row is loaded
+// before this one's rounds.
+//
+// settle: the rule for a warp's 32 consecutive vertices, each with the mask m
+// of the colours of its neighbours outside the group and the bits wmask of its
+// lower neighbours in it; c holds the current colours and receives the exact
+// ones. At most kWarpTries evaluations of all lanes at once, each against the
+// current colours (one suffices where nothing changes), else lane by lane.
+// Returns false if a lane meets a colour that M has no bit for.
+constexpr int kWarpTries = 3;
+template <class M>
+__device__ __forceinline__ bool settle(M m, uint32_t wmask, uint32_t steps, bool live, uint32_t& c) {
+    constexpr uint32_t kBits = sizeof(M) == 8 ? 64 : 31;  // 32-bit masks keep bit 31 for the colours above 30
+    auto mex = [](M x) { return sizeof(M) == 8 ? (uint32_t)__ffsll((long long)~x) - 1 : (uint32_t)__ffs((int)~x) - 1; };
+    for (int tries = 0; tries < kWarpTries; ++tries) {
+        M mw = m;
+        bool out = false;
+        uint32_t b = wmask;
+        for (uint32_t k = 0; k < steps; ++k, b &= b - 1u) {
+            const uint32_t cu = __shfl_sync(0xffffffffu, c, b ? __ffs((int)b) - 1 : 0);
+            if (b && cu < kBits) mw |= (M)1 << cu;
+            out = out || (b && cu >= kBits);
+        }
+        if (__any_sync(0xffffffffu, live && (out || mex(mw) >= kBits))) return false;
+        const uint32_t cn = mex(mw);
+        const bool same = !__any_sync(0xffffffffu, live && cn != c);
+        if (live) c = cn;
+        if (same) return true;
+    }
+    // lane k's colour is exact once those of lanes 0..k-1 are; a lane out of bits is found at the end
+    M mw = m;
+    for (uint32_t b = __reduce_or_sync(0xffffffffu, wmask); b; b &= b - 1u) {
+        const uint32_t k = __ffs((int)b) - 1;
+        const uint32_t ck = __shfl_sync(0xffffffffu, mex(mw), k);
+        if ((wmask >> k & 1u) && ck < kBits) mw |= (M)1 << ck;
+    }
+    if (__any_sync(0xffffffffu, live && mex(mw) >= kBits)) return false;
+    if (live) c = mex(mw);
+    return true;
+}
+
+// The same where every lane's only neighbour in its group is the lane before it
+// (or none), as in a row-major grid whose rows are longer than a warp: lane k's
+// rule is then a function of one colour, x -> b if x == a else a, with a and b
+// the first and second colour free of m. Such functions compose into (key, value
+// if equal, value if not), so a prefix scan of five shuffles gives every lane's
+// colour, ~250 cycles where lane by lane takes ~1,900. m: colours below 31.
+// Returns false if a lane's colour may exceed 30.
+__device__ __forceinline__ bool settle_chain(uint32_t m, uint32_t wmask, bool live, uint32_t& c) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t fa = ~m & (m + 1u), rest = m | fa, fb = ~rest & (rest + 1u);  // lowest clear bits
+    const uint32_t a = (uint32_t)__ffs((int)fa) - 1, b = (uint32_t)__ffs((int)fb) - 1;
+    if (__any_sync(0xffffffffu, live && rest >= 0x7fffffffu)) return false;  // the second free colour is above 30
+    uint32_t key = wmask ? a : 255u, eq = wmask ? b : a, ne = a;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, key | eq << 8 | ne << 16, d);
+        if (lane >= (uint32_t)d) {
+            const uint32_t oe = o >> 8 & 255u, on = o >> 16 & 255u;
+            const uint32_t e = oe == key ? eq : ne, n = on == key ? eq : ne;
+            key = o & 255u;
+            eq = e;
+            ne = n;
+        }
+    }
+    if (live) c = ne;  // lane 0's function is constant, and so is every composition from it on
+    return true;
+}
+
+constexpr int kAhead = 8;       // row entries loaded ahead
+constexpr uint32_t kSmemColors = 90 * 1024;  // 180 KB of uint16 colours
+// Dynamic shared memory: the colours (n <= kSmemColors) and, in what is left, a
+// row of kChunk chunk-local indices for each of `inner_cap` in-chunk
+// neighbours per vertex (17 at n = 92,160, 32 below 76k vertices and where the
+// colours stay in global memory); further neighbours are read from the row.
+constexpr int kMaxInner = 32;
+constexpr size_t kWalkSmem = 214 * 1024;  // + 12 KB static
+inline int walk_inner_cap(size_t color_bytes) {
+    return (int)std::min<size_t>(kMaxInner, (kWalkSmem - color_bytes) / (kChunk * sizeof(uint16_t)));
+}
+__global__ void __launch_bounds__(kChunk) k_color_walk(ColorView g, ColorRows r, uint16_t* col_g,
+                                                      const unsigned int* first, unsigned int* rounds_out,
+                                                      unsigned int* err, uint32_t inner_cap) {
+    extern __shared__ uint16_t walk_s[];
+    uint16_t* inner = walk_s + threadIdx.x;  // [inner_cap][kChunk], this thread's column
+    uint16_t* col_s = walk_s + inner_cap * kChunk;
+    __shared__ uint16_t chunk_col[2][kChunk];   // the chunk's colours: the last round's and this one's
+    // bit c of a colour c < 31, bit 31 for the others: what most rounds need
+    __shared__ uint32_t chunk_bit[2][kChunk];
+    __shared__ unsigned warp_changed[3];        // warps with a changed colour: this round's, the last one's, the next one's
+    const uint32_t start = *first;
+    const uint32_t t = threadIdx.x;
     if (start >= g.n) {  // already a fixed point
-        if (threadIdx.x == 0) *rounds_out = 0;
+        if (t == 0) *rounds_out = 0;
         return;
     }
-    bool smem = g.n <= kSmemColors;
+    const uint32_t chunk0 = start & ~(uint32_t)(kChunk - 1);
+    const bool smem = g.n <= kSmemColors;
     uint16_t* col = col_g;
     if (smem) {
-        for (uint32_t i = threadIdx.x; i < g.n; i += kChunk) col_s[i] = col_g[i];
-        __syncthreads();
+        for (uint32_t i = t; i < g.n; i += kChunk) col_s[i] = col_g[i];
         col = col_s;
     }
-    const uint32_t t = threadIdx.x;
+    // this chunk's rows: their first entries loaded one chunk ahead, their heads two
+    uint4 head = make_uint4(0u, 0u, 0u, 0u), next_head = head;
+    uint4 ahead_a = head, ahead_b = head;
+    auto load_head = [&](uint32_t v) { return v < g.n ? r.head[v] : make_uint4(0u, 0u, 0u, 0u); };
+    auto load_row = [&](uint4 h) {
+        // 16-byte aligned; a row may have fewer than kAhead entries, the buffer is padded past its end
+        const uint4* row = reinterpret_cast<const uint4*>(r.adj) + h.x;
+        ahead_a = row[0];
+        ahead_b = row[1];
+    };
+    head = load_head(chunk0 + t);
+    next_head = load_head(chunk0 + kChunk + t);
+    load_row(head);
+    if (t < 3) warp_changed[t] = 0u;
+    __syncthreads();
     unsigned int rounds = 0;
-    for (uint32_t base = (start / kChunk) * kChunk; base < g.n; base += kChunk) {
+    for (uint32_t base = chunk0; base < g.n; base += kChunk) {
         const uint32_t v = base + t;
         const bool live = v < g.n;
-        // set-up: final colours below the chunk into a mask, in-chunk lower
-        // neighbours into shared memory
+        const bool slow = head.y == kRowSlow;
+        const uint32_t n_out = slow ? 0u : (head.y & 0xffffu), n_in = slow ? 0u : (head.y >> 16);
+        const uint32_t n_row = n_out + n_in, n_kept = min(n_in, inner_cap);
+        const uint32_t wmask = head.z;
+        const uint32_t* my_row = r.adj + 4 * (size_t)head.x;
+        const uint32_t steps = __reduce_max_sync(0xffffffffu, (uint32_t)__popc(wmask));
+        // final colours below the chunk into a mask, in-chunk neighbours into shared memory
         unsigned long long outer = 0;
-        bool slow = false;
-        uint32_t ninner = 0;
-        auto visit = [&](uint32_t u) {
-            if (u >= v) return;
-            if (u < base) {
-                mark(outer, col[u], slow);
-            } else if (ninner < kInner) {
-                inner[ninner++][t] = (uint16_t)(u - base);
+        bool outer_high = slow;
+        unsigned depends = slow ? ~0u : 0u;  // warps of this chunk that the colours depend on (all, without a row)
+        auto take = [&](uint32_t k, uint32_t u) {
+            if (k < n_out) {
+                mark(outer, col[u], outer_high);
             } else {
-                slow = true;
+                const uint32_t i = u - base, j = k - n_out;
+                if (j < n_kept) inner[j * kChunk] = (uint16_t)i;
+                depends |= 1u << (i >> 5);
             }
         };
-        if (live) {
-            for (uint32_t k = g.lo_off[v]; k < g.lo_off[v + 1]; ++k) visit(g.lo[k]);
-            for (uint32_t k = g.contacts.inc_off[v]; k < g.contacts.inc_off[v + 1]; ++k) {
-                uint32_t c = g.contacts.inc[k];
-                uint32_t kind = g.contacts.kind[c];
-                uint4 cv = g.contacts.verts[c];
-                uint32_t ids[4] = {cv.x, cv.y, cv.z, cv.w};
-                uint32_t cnt = kind == 0 ? 2u : (kind == 1 ? 3u : 4u);
-                for (uint32_t j = 0; j < cnt; ++j) visit(ids[j]);
-            }
-            if (g.grab_active && (g.grab_v[0] == v || g.grab_v[1] == v || g.grab_v[2] == v))
-                for (int j = 0; j < 3; ++j) visit(g.grab_v[j]);
-            chunk_col[t] = col[v];
-        }
+        const uint32_t ahead[kAhead] = {ahead_a.x, ahead_a.y, ahead_a.z, ahead_a.w,
+                                        ahead_b.x, ahead_b.y, ahead_b.z, ahead_b.w};
+#pragma unroll
+        for (uint32_t k = 0; k < kAhead; ++k)
+            if (k < n_row) take(k, ahead[k]);
+#pragma unroll 4
+        for (uint32_t k = kAhead; k < n_row; ++k) take(k, my_row[k]);
+        depends = __reduce_or_sync(0xffffffffu, depends);
+        const bool chain = __all_sync(0xffffffffu, (wmask & ~(t & 31u ? 1u << ((t & 31u) - 1u) : 0u)) == 0u);
+        const uint32_t outer32 = (uint32_t)(outer & 0x7fffffffull) | ((outer >> 31) != 0ull || outer_high ? 1u << 31 : 0u);
+        uint32_t cur = live ? col[v] : 0u;
+        auto bit_of = [](uint32_t c) { return 1u << min(c, 31u); };
+        chunk_col[0][t] = (uint16_t)cur;
+        chunk_bit[0][t] = bit_of(cur);
+        head = next_head;
+        if (base + kChunk < g.n) load_row(head);
+        next_head = load_head(v + 2 * kChunk);
         __syncthreads();
-        int r = 0;
-        for (; r <= kChunk + 1; ++r) {
-            uint32_t c = 0u;
-            if (live) {
-                unsigned long long mask = outer;
-                bool high = slow;
-                for (uint32_t j = 0; j < ninner; ++j) mark(mask, chunk_col[inner[j][t]], high);
-                // colours >= 64 around v, or all of 0..63 taken: the full rule
-                if (high || ~mask == 0ull) c = greedy_color(g, col, v);
-                else c = (uint32_t)__ffsll((long long)~mask) - 1;
+        int rd = 0, buf = 0;
+        bool again = true;  // this warp has not settled: the first round, or it took the full rule
+        uint32_t m_last = 0;
+        for (; rd <= kChunk + 1; ++rd) {
+            const uint16_t* now = chunk_col[buf];
+            auto color_of = [&](uint32_t u) { return (uint32_t)(u >= base ? now[u - base] : col[u]); };
+            uint32_t c = cur;
+            const unsigned slot = rounds % 3;  // goes on over the chunks
+            if (t == 0) warp_changed[(slot + 1) % 3] = 0u;  // last read in the last round
+            if (again || (depends & warp_changed[(slot + 2) % 3])) {
+                const uint32_t* bits = chunk_bit[buf];
+                uint32_t m = outer32;
+#pragma unroll 4
+                for (uint32_t j = 0; j < n_kept; ++j) m |= bits[inner[j * kChunk]];
+                for (uint32_t j = n_kept; j < n_in; ++j) m |= bits[my_row[n_out + j] - base];
+                // nothing to do where the warp had settled and no lane's outside mask moved
+                const bool wide = __any_sync(0xffffffffu, live && m >> 31);
+                const bool moved = again || wide || __any_sync(0xffffffffu, live && m != m_last);
+                m_last = m;
+                bool full = false;
+                unsigned long long m64 = outer;
+                bool high = outer_high;
+                if (moved && (wide || !(chain ? settle_chain(m, wmask, live, c)
+                                              : settle<uint32_t>(m, wmask, steps, live, c)))) {
+                    // colours above 30 around: 64-bit masks
+                    for (uint32_t j = 0; j < n_in; ++j)
+                        mark(m64, now[j < n_kept ? (uint32_t)inner[j * kChunk] : my_row[n_out + j] - base], high);
+                    c = cur;
+                    full = __any_sync(0xffffffffu, live && high) ||
+                           !settle<unsigned long long>(m64, wmask, steps, live, c);
+                }
+                if (full && live) {
+                    // a lane has no row or meets colours >= 64: the whole warp takes the rule on the last round's colours
+                    unsigned long long ml = m64;
+                    bool hl = high;
+                    for (uint32_t b = wmask; b; b &= b - 1u) mark(ml, now[(t & ~31u) + __ffs((int)b) - 1], hl);
+                    c = (hl || ~ml == 0ull) ? greedy_color(g, v, color_of) : (uint32_t)__ffsll((long long)~ml) - 1;
+                }
+                again = full;
             }
-            __syncthreads();
-            int changed = (live && c != chunk_col[t]) ? 1 : 0;
+            const bool changed = live && c != cur;
             if (changed) {
-                chunk_col[t] = (uint16_t)c;
+                cur = c;
                 col[v] = (uint16_t)c;
             }
+            chunk_col[buf ^ 1][t] = (uint16_t)cur;
+            chunk_bit[buf ^ 1][t] = bit_of(cur);
+            buf ^= 1;
             ++rounds;
-            if (!__syncthreads_or(changed)) break;
+            if (__any_sync(0xffffffffu, changed) && (t & 31u) == 0) atomicOr(&warp_changed[slot], 1u << (t >> 5));
+            __syncthreads();
+            if (!warp_changed[slot]) break;
         }
-        if (r > kChunk + 1 && t == 0) atomicOr(err, 1u);
+        if (rd > kChunk + 1 && t == 0) atomicOr(err, 1u);
     }
-    if (smem) {
-        __syncthreads();
-        for (uint32_t i = (start / kChunk) * kChunk + threadIdx.x; i < g.n; i += kChunk) col_g[i] = col_s[i];
-    }
+    if (smem)
+        for (uint32_t i = chunk0 + t; i < g.n; i += kChunk) col_g[i] = col_s[i];
     if (t == 0) *rounds_out = rounds;
 }
 
-// Lowest vertex whose greedy rule fails for the current colouring.
-__global__ void k_color_probe(ColorView g, const uint16_t* col, unsigned int* first) {
-    unsigned int lo = 0xffffffffu;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n; v += gridDim.x * blockDim.x)
-        if (greedy_color(g, col, v) != col[v]) lo = min(lo, v);
-    for (int o = 16; o > 0; o >>= 1) lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    if ((threadIdx.x & 31) == 0 && lo != 0xffffffffu) atomicMin(first, lo);
-}
-
-__global__ void k_color_count(uint32_t n, const uint16_t* col, uint32_t* counts) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        atomicAdd(&counts[col[v]], 1u);
+// Vertices per colour: counted per block in shared memory (atomics on a few
+// global counters took 23 us on the fold, 322 us on a 1024 x 1024 sheet).
+__global__ void __launch_bounds__(256) k_color_count(uint32_t n, const uint16_t* col, uint32_t* counts) {
+    constexpr uint32_t kLocal = 64;
+    __shared__ uint32_t local[kLocal];
+    if (threadIdx.x < kLocal) local[threadIdx.x] = 0u;
+    __syncthreads();
+    const uint32_t stride = gridDim.x * 256;
+    for (uint32_t v0 = blockIdx.x * 256; v0 < n; v0 += stride) {
+        const uint32_t v = v0 + threadIdx.x;
+        const uint32_t c = v < n ? col[v] : ~0u;
+        const unsigned same = __match_any_sync(0xffffffffu, c);
+        if (v < n && (threadIdx.x & 31u) == (uint32_t)__ffs((int)same) - 1) {
+            const uint32_t k = (uint32_t)__popc(same);
+            if (c < kLocal) atomicAdd(&local[c], k);
+            else atomicAdd(&counts[c], k);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < kLocal && local[threadIdx.x]) atomicAdd(&counts[threadIdx.x], local[threadIdx.x]);
 }
 
 __global__ void k_iota(uint32_t n, uint32_t* out) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) out[v] = v;
 }
 
-void Coloring::init(uint32_t n, cudaStream_t s) {
+void Coloring::init(uint32_t n, uint64_t lo_total, cudaStream_t s) {
     n_ = n;
+    lo_total_ = lo_total;
+    row_head_.reserve(n);
     a_.reserve(n);
     b_.reserve(n);
     order_.reserve(n);
@@ -207,14 +472,19 @@ void Coloring::compute(const ColorView& view, cudaStream_t s) {
     // first vertex the probe finds out of date
     CC_CUDA(cudaMemsetAsync(changed_.ptr, 0, 2 * sizeof(unsigned int), s));
     CC_CUDA(cudaMemsetAsync(changed_.ptr + 2, 0xff, sizeof(unsigned int), s));
-    k_color_probe<<<grid_for(n, 256), 256, 0, s>>>(view, cur_, changed_.ptr + 2);
-    size_t smem = n <= kSmemColors ? n * sizeof(uint16_t) : 0;
-    allow_dynamic_smem(k_color_chunked, smem);
-    k_color_chunked<<<1, kChunk, smem, s>>>(view, cur_, changed_.ptr + 2, changed_.ptr, changed_.ptr + 1);
+    adj_.reserve(row_bound(lo_total_, view.n_incident, n) + 3 + kAhead);
+    ColorRows rows{adj_.ptr, row_head_.ptr};
+    k_color_rows<<<grid_for((size_t)n * kRowLanes, 128), 128, 0, s>>>(view, rows, cur_, changed_.ptr + 2);
+    const size_t color_bytes = n <= kSmemColors ? n * sizeof(uint16_t) : 0;
+    const int inner_cap = walk_inner_cap(color_bytes);
+    const size_t smem = inner_cap * kChunk * sizeof(uint16_t) + color_bytes;
+    CC_CUDA(cudaFuncSetAttribute((const void*)k_color_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem));
+    k_color_walk<<<1, kChunk, smem, s>>>(view, rows, cur_, changed_.ptr + 2, changed_.ptr, changed_.ptr + 1,
+                                         (uint32_t)inner_cap);
     launches_ += 2;
     CC_CUDA(cudaGetLastError());
     CC_CUDA(cudaMemsetAsync(counts_.ptr, 0, kMaxColors * sizeof(uint32_t), s));
-    k_color_count<<<grid_for(n, 256), 256, 0, s>>>(n, cur_, counts_.ptr);
+    k_color_count<<<std::min(grid_for(n, 256), 148 * 2), 256, 0, s>>>(n, cur_, counts_.ptr);
     CC_CUDA(cudaMemcpyAsync(counts_h_.ptr, counts_.ptr, kMaxColors * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     CC_CUDA(cudaMemcpyAsync(changed_h_.ptr, changed_.ptr, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
     CC_CUDA(cudaStreamSynchronize(s));

@@ -11,13 +11,15 @@ struct ColorView {
     const uint32_t* lo_off;  // [n+1] lower-index neighbours of the material graph
     const uint32_t* lo;
     ContactsView contacts;
+    uint64_t n_incident;  // entries of contacts.inc
     int grab_active;
     uint32_t grab_v[3];
 };
 
 class Coloring {
    public:
-    void init(uint32_t n, cudaStream_t s);
+    // lo_total: entries of the material graph's lower-neighbour lists
+    void init(uint32_t n, uint64_t lo_total, cudaStream_t s);
     // Recompute the colouring for the current graph, starting from the last one.
     void compute(const ColorView& view, cudaStream_t s);
     uint32_t n_colors() const { return n_colors_; }
@@ -33,6 +35,9 @@ class Coloring {
    private:
     static constexpr int kBatch = 8;
     uint32_t n_ = 0;
+    uint64_t lo_total_ = 0;
+    DBuf<uint32_t> adj_;   // distinct lower neighbours of every vertex (k_color_rows)
+    DBuf<uint4> row_head_;
     DBuf<uint16_t> a_, b_;
     uint16_t* cur_ = nullptr;
     DBuf<uint32_t> order_, counts_, iota_;

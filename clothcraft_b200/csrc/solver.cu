@@ -565,6 +565,7 @@ struct cc_solver {
         c.lo_off = lo_off.ptr;
         c.lo = lo.ptr;
         c.contacts = cv;
+        c.n_incident = world->stats().n_incident;
         c.grab_active = grab ? 1 : 0;
         if (grab)
             for (int k = 0; k < 3; ++k) c.grab_v[k] = grab->vertices[k];
@@ -1419,7 +1420,7 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
         h->ext_w_s.reserve(T);
         h->ext_cum.reserve(T);
         h->residual.zero(n, st);
-        h->coloring.init((uint32_t)n, st);
+        h->coloring.init((uint32_t)n, lo_v.size(), st);
         // initial state
         for (uint64_t i = 0; i < n; ++i) {
             h->stage.ptr[i] = make_double4(x0[3 * i], x0[3 * i + 1], x0[3 * i + 2], 0.0);
