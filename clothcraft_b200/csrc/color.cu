@@ -272,10 +272,13 @@ constexpr uint32_t kSmemColors = 90 * 1024;  // 180 KB of uint16 colours
 // Dynamic shared memory: the colours (n <= kSmemColors) and, in what is left, a
 // row of kChunk chunk-local indices for each of `inner_cap` in-chunk
 // neighbours per vertex (17 at n = 92,160, 32 below 76k vertices and where the
-// colours stay in global memory); further neighbours are read from the row.
+// colours stay in global memory); further neighbours are read from the row. Up
+// to four chunks take 12, which keeps the block below 48 KB: a step of a few
+// dozen launches feels the SM's change to a large shared-memory carve-out.
 constexpr int kMaxInner = 32;
 constexpr size_t kWalkSmem = 214 * 1024;  // + 12 KB static
-inline int walk_inner_cap(size_t color_bytes) {
+inline int walk_inner_cap(uint32_t n, size_t color_bytes) {
+    if (n <= 4 * kChunk) return 12;
     return (int)std::min<size_t>(kMaxInner, (kWalkSmem - color_bytes) / (kChunk * sizeof(uint16_t)));
 }
 __global__ void __launch_bounds__(kChunk) k_color_walk(ColorView g, ColorRows r, uint16_t* col_g,
@@ -476,9 +479,10 @@ void Coloring::compute(const ColorView& view, cudaStream_t s) {
     ColorRows rows{adj_.ptr, row_head_.ptr};
     k_color_rows<<<grid_for((size_t)n * kRowLanes, 128), 128, 0, s>>>(view, rows, cur_, changed_.ptr + 2);
     const size_t color_bytes = n <= kSmemColors ? n * sizeof(uint16_t) : 0;
-    const int inner_cap = walk_inner_cap(color_bytes);
+    const int inner_cap = walk_inner_cap(n, color_bytes);
     const size_t smem = inner_cap * kChunk * sizeof(uint16_t) + color_bytes;
-    CC_CUDA(cudaFuncSetAttribute((const void*)k_color_walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem));
+    static std::atomic<uint64_t> raised{0};  // devices on which the limit is raised
+    allow_dynamic_smem_once(k_color_walk, kWalkSmem, raised);
     k_color_walk<<<1, kChunk, smem, s>>>(view, rows, cur_, changed_.ptr + 2, changed_.ptr, changed_.ptr + 1,
                                          (uint32_t)inner_cap);
     launches_ += 2;

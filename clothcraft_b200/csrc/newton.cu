@@ -32,6 +32,7 @@ constexpr int kBlocks = kSumBlocks;
 // g_out[3v..3v+2] = dE/dx_v at s.x for moving vertex v (0 where pinned)
 template <int G>
 __global__ void __launch_bounds__(128) k_nt_gradient(SweepView s, double* g_out) {
+    __shared__ double near_s[128 / G * Near<G>::kDoubles];
     uint32_t t = blockIdx.x * 128 + threadIdx.x;
     uint32_t v = t / G;
     if (v >= s.n) return;
@@ -45,7 +46,10 @@ __global__ void __launch_bounds__(128) k_nt_gradient(SweepView s, double* g_out)
     d3 g = mk(0, 0, 0);
     Sym H;
     sym_zero(H);
-    local_part<true, G, false>(s, v, x, lane, g, H);
+    Near<G> T;
+    T.head(s, v);
+    const typename Near<G>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
+    local_part<true, G, false>(s, T, f, x, lane, g, H);
     if (G > 1) {
         g.x = group_sum<G>(g.x, mask);
         g.y = group_sum<G>(g.y, mask);
@@ -61,21 +65,30 @@ __global__ void __launch_bounds__(128) k_nt_gradient(SweepView s, double* g_out)
 
 // Jacobi diagonal of System::diagonal (src/solver.rs:150-161): inertia +
 // shift + the diagonal of every incident term's Hessian; 1 on fixed dofs.
-__global__ void k_nt_diagonal(SweepView s, double shift, double* diag) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < s.n; v += gridDim.x * blockDim.x) {
+template <int G>
+__global__ void __launch_bounds__(128) k_nt_diagonal(SweepView s, double shift, double* diag) {
+    __shared__ double near_s[128 / G * Near<G>::kDoubles];
+    const uint32_t lane = threadIdx.x & (G - 1);
+    const unsigned mask = ((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1));
+    for (uint32_t v = (blockIdx.x * 128 + threadIdx.x) / G; v < s.n; v += gridDim.x * 128 / G) {
         if (s.pinned[v]) {
-            diag[3 * v] = diag[3 * v + 1] = diag[3 * v + 2] = 1.0;
+            if (lane == 0) diag[3 * v] = diag[3 * v + 1] = diag[3 * v + 2] = 1.0;
             continue;
         }
         d3 x = ld3(s.x, v);
+        Near<G> T;
+        T.head(s, v);
+        const typename Near<G>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
         d3 g = mk(0, 0, 0);
         Sym H;
         sym_zero(H);
-        local_part<true, 1>(s, v, x, 0, g, H);
+        local_part<true, G>(s, T, f, x, lane, g, H);
+        const double hx = group_sum<G>(H.a[0], mask), hy = group_sum<G>(H.a[3], mask), hz = group_sum<G>(H.a[5], mask);
+        if (lane != 0) continue;
         double m = s.inertia[v];
-        diag[3 * v] = fmax(H.a[0] + m + shift, 1e-12);
-        diag[3 * v + 1] = fmax(H.a[3] + m + shift, 1e-12);
-        diag[3 * v + 2] = fmax(H.a[5] + m + shift, 1e-12);
+        diag[3 * v] = fmax(hx + m + shift, 1e-12);
+        diag[3 * v + 1] = fmax(hy + m + shift, 1e-12);
+        diag[3 * v + 2] = fmax(hz + m + shift, 1e-12);
     }
 }
 
@@ -260,7 +273,7 @@ class Newton {
     void diagonal(double shift) {
         SweepView s = pb_.view;
         s.x = w_.x.ptr;
-        k_nt_diagonal<<<grid_for(s.n, 128), 128, 0, st_>>>(s, shift, w_.diag.ptr);
+        k_nt_diagonal<kLanes><<<grid_for(kLanes * (size_t)s.n, 128), 128, 0, st_>>>(s, shift, w_.diag.ptr);
     }
     double read_scalar() {
         CC_CUDA(cudaMemcpyAsync(w_.h_scalar.ptr, w_.scalars.ptr, sizeof(double), cudaMemcpyDeviceToHost, st_));

@@ -444,6 +444,13 @@ struct cc_solver {
     DBuf<double> st_w, st_k;
     DBuf<uint32_t> inc_off, inc, lo_off, lo;
     DBuf<uint2> inc_mid;  // per vertex: first hinge entry, first stitch entry
+    // per-vertex records of the elastic terms (VertexTerms)
+    DBuf<uint4> vt_head;
+    DBuf<uint32_t> vt_nb;
+    DBuf<unsigned long long> vt_tri;
+    DBuf<double4> vt_tri_b, vt_tri_k;
+    DBuf<ulonglong2> vt_hinge;
+    DBuf<uint4> vt_heads;  // in colour order, of the last colouring
     DBuf<uint8_t> pinned;
     DBuf<double> masses;
     // state and per-step buffers
@@ -542,6 +549,7 @@ struct cc_solver {
         v.st_v = st_v.ptr;
         v.st_w = st_w.ptr;
         v.st_k = st_k.ptr;
+        v.vt = {vt_head.ptr, vt_nb.ptr, vt_tri.ptr, vt_tri_b.ptr, vt_tri_k.ptr, vt_hinge.ptr};
         v.contacts = cv;
         v.contact_r = s.contact.radius;
         v.contact_k = s.contact.stiffness;
@@ -661,8 +669,13 @@ struct cc_solver {
         return r;
     }
     void launch_variant(const SweepView& sv, const uint32_t* order, uint32_t count, int variant, bool fp32) {
-        if (fp32) launch_sweep32(sv, order, count, variant, stream, grid_cap(variant, true));
-        else launch_sweep(sv, order, count, variant, stream, grid_cap(variant, false));
+        if (fp32) {
+            launch_sweep32(sv, order, count, variant, stream, grid_cap(variant, true));
+        } else {
+            SweepView c = sv;
+            c.heads = vt_heads.ptr + 3 * (order - coloring.order());
+            launch_sweep(c, count, variant, stream, grid_cap(variant, false));
+        }
     }
     void sweep(const SweepView& sv, const uint32_t* order, uint32_t count, bool fp32) {
         launch_variant(sv, order, count, fp32 ? lanes32 : lanes, fp32);
@@ -721,6 +734,9 @@ struct cc_solver {
         double t = now_ms();
         coloring.set_error_word(&sc.ptr->error);
         coloring.compute(color_view(cv, grab), stream);
+        vt_heads.reserve(3 * (size_t)n);
+        launch_color_heads(sweep_view(cv, cc_vbd_settings{}, nullptr), coloring.order(), vt_heads.ptr, stream);
+        ++own_launches;
         m.color_ms += now_ms() - t;
         m.color_rounds += coloring.last_iterations();
     }
@@ -1265,7 +1281,7 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
             const cc_material& M = mesh->materials[k];
             mats.push_back({M.warp, M.weft, M.shear, M.compression_ratio, M.compression_transition});
         }
-        if (mats.empty()) throw Failure{CC_ERR_INVALID_ARGUMENT, "Invalid material binding or mesh topology"};
+        if (mats.empty() || mats.size() >> 22) throw Failure{CC_ERR_INVALID_ARGUMENT, "Invalid material binding or mesh topology"};
         auto grain = [&](uint32_t mat, double& sn, double& cs) {
             double r = mesh->materials[mat].grain_degrees * (M_PI / 180.0);
             sn = std::sin(r);
@@ -1337,16 +1353,26 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
         }
         std::vector<uint32_t> io(n + 1, 0), iv, lo_o(n + 1, 0), lo_v;
         std::vector<uint2> mid(n);
+        std::vector<uint4> head(2 * n);
+        std::vector<uint32_t> nb;
+        uint32_t n_vt_tri = 0, n_vt_hinge = 0;
         for (uint64_t v = 0; v < n; ++v) {
             io[v + 1] = io[v] + (uint32_t)inc[v].size();
             // entries are grouped by type (triangles, hinges, stitches): record the boundaries
-            uint32_t hb = io[v], sb = io[v];
+            uint32_t hb = io[v], sb = io[v], ends = 0;
             for (uint32_t e : inc[v]) {
                 uint32_t type = e >> 30;
                 if (type == TERM_TRI) ++hb, ++sb;
-                else if (type == TERM_HINGE) ++sb;
+                else if (type == TERM_HINGE) ++sb, ends += ((e >> 28) & 3u) < 2u ? 1u : 0u;
             }
             mid[v] = make_uint2(hb, sb);
+            head[2 * v] = make_uint4((uint32_t)nb.size(), (uint32_t)graph[v].size(), n_vt_tri, hb - io[v]);
+            head[2 * v + 1] = make_uint4(n_vt_hinge, ends, sb - hb - ends, io[v + 1] - sb);
+            if (graph[v].size() >> 21)  // the records' 21-bit places
+                throw Failure{CC_ERR_INVALID_ARGUMENT, "a vertex has more than 2^21 mesh neighbours"};
+            nb.insert(nb.end(), graph[v].begin(), graph[v].end());
+            n_vt_tri += hb - io[v];
+            n_vt_hinge += sb - hb;
             iv.insert(iv.end(), inc[v].begin(), inc[v].end());
             for (uint32_t u : graph[v])
                 if (u < v) lo_v.push_back(u);
@@ -1389,6 +1415,17 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
         h->inc_off.upload(io, st);
         h->inc_mid.upload(mid, st);
         h->inc.upload(iv, st);
+        h->vt_head.upload(head, st);
+        h->vt_nb.upload(nb, st);
+        h->vt_tri.reserve(n_vt_tri);
+        h->vt_tri_b.reserve(n_vt_tri);
+        h->vt_tri_k.reserve(n_vt_tri);
+        h->vt_hinge.reserve(n_vt_hinge);
+        {
+            const cc_vbd_settings none{};
+            launch_vertex_terms(h->sweep_view(h->world->contacts(), none, nullptr), h->vt_tri.ptr, h->vt_tri_b.ptr,
+                                h->vt_tri_k.ptr, h->vt_hinge.ptr, st);
+        }
         h->lo_off.upload(lo_o, st);
         h->lo.upload(lo_v, st);
         h->pinned.upload(pin, st);

@@ -24,21 +24,25 @@
 namespace cc {
 
 template <int G>
-__device__ __forceinline__ void solve_vertex(const SweepView& s, uint32_t v, uint32_t lane, unsigned mask) {
-    if (s.pinned[v]) {
+__device__ __forceinline__ void solve_vertex(const SweepView& s, uint32_t i, uint32_t lane, unsigned mask, double* smem) {
+    Near<G> T;
+    T.head_of_color(s, i);
+    const uint32_t v = T.v;
+    if (T.nt == kPinnedHead) {
         if (lane == 0) s.residual[v] = 0.0;
         return;
     }
-    d3 x = ld3(s.x, v);
-    d3 y = ld3(s.target, v);
-    double m = s.inertia[v];
+    // everything that the vertex's number leads to, before the first of it is waited for
+    const d3 x = ld3(s.x, v);
+    const d3 y = ld3(s.target, v);
+    const double m = s.inertia[v];
+    const d3 ctr = ld3(s.contacts.centers, v);
+    const double rad = s.contacts.radii[v];
+    const typename Near<G>::First f = T.load(s, lane, mask, smem);
     d3 g = mk(0, 0, 0);
     Sym H;
     sym_zero(H);
-    double e_el = local_part<true, G>(s, v, x, lane, g, H);
-    // the OGC ball, loaded here so that its latency hides behind the reductions
-    const d3 ctr = ld3(s.contacts.centers, v);
-    const double rad = s.contacts.radii[v];
+    double e_el = local_part<true, G>(s, T, f, x, lane, g, H);
     if (G > 1) {
         e_el = group_sum<G>(e_el, mask);
         g.x = group_sum<G>(g.x, mask);
@@ -82,7 +86,7 @@ __device__ __forceinline__ void solve_vertex(const SweepView& s, uint32_t v, uin
         truncated = truncated || bound;
         d3 gd;
         Sym Hd;
-        double e = local_part<false, G>(s, v, cand, lane, gd, Hd);
+        double e = local_part<false, G>(s, T, T.first(s, lane), cand, lane, gd, Hd);
         if (G > 1) e = group_sum<G>(e, mask);
         d3 cy = cand - y;
         e += 0.5 * m * dot(cy, cy);
@@ -103,24 +107,25 @@ __device__ __forceinline__ void solve_vertex(const SweepView& s, uint32_t v, uin
 // Each group of G lanes solves vertices gi, gi + groups in the grid, ...: one
 // vertex per group when the grid covers the colour, several in a persistent grid.
 template <int G, int BLOCK, int MINB>
-__global__ void __launch_bounds__(BLOCK, MINB) k_sweep(SweepView s, const uint32_t* order, uint32_t count) {
+__global__ void __launch_bounds__(BLOCK, MINB) k_sweep(SweepView s, uint32_t count) {
+    constexpr uint32_t kGroups = BLOCK / G;
+    __shared__ double near_s[kGroups * Near<G>::kDoubles];
     if (s.skip_at && *s.skip_at <= s.iteration) return;  // a refresh detection precedes this iteration
     const uint32_t lane = threadIdx.x & (G - 1);
     const unsigned mask = G >= 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1)));
-    constexpr uint32_t kGroups = BLOCK / G;
     stamp_block_start(s);
     // whole groups step together
     for (uint32_t gi = blockIdx.x * kGroups + threadIdx.x / G; gi < count; gi += gridDim.x * kGroups)
-        solve_vertex<G>(s, order[gi], lane, mask);
+        solve_vertex<G>(s, gi, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
     stamp_block_end(s);
 }
 
 template <int G, int B, int MINB>
-static void launch_k(const SweepView& s, const uint32_t* order, uint32_t count, cudaStream_t st, unsigned cap) {
+static void launch_k(const SweepView& s, uint32_t count, cudaStream_t st, unsigned cap) {
     uint64_t threads = (uint64_t)count * G;
     unsigned grid = (unsigned)((threads + B - 1) / B);
     if (cap && grid > cap) grid = cap;
-    k_sweep<G, B, MINB><<<grid, B, 0, st>>>(s, order, count);
+    k_sweep<G, B, MINB><<<grid, B, 0, st>>>(s, count);
 }
 
 template <int G, int B, int MINB>
@@ -184,13 +189,12 @@ bool sweep_variant_valid(int variant, bool fp32) {
 namespace {
 struct SweepLaunch {
     const SweepView& s;
-    const uint32_t* order;
     uint32_t count;
     cudaStream_t st;
     unsigned cap;
     template <int G, int B, int MINB>
     int operator()() const {
-        launch_k<G, B, MINB>(s, order, count, st, cap);
+        launch_k<G, B, MINB>(s, count, st, cap);
         return 0;
     }
 };
@@ -202,24 +206,33 @@ struct SweepResident {
 };
 }  // namespace
 
-void launch_sweep(const SweepView& s, const uint32_t* order, uint32_t count, int variant, cudaStream_t st,
-                  unsigned grid_cap) {
+void launch_sweep(const SweepView& s, uint32_t count, int variant, cudaStream_t st, unsigned grid_cap) {
     if (count == 0) return;
     SweepVariant v = decode_variant(variant);
-    dispatch(v, SweepLaunch{s, order, count, st, v.persistent ? grid_cap : 0u});
+    dispatch(v, SweepLaunch{s, count, st, v.persistent ? grid_cap : 0u});
 }
 
 unsigned sweep_resident_blocks(int variant) { return dispatch(decode_variant(variant), SweepResident{}); }
 
 // Probe: local e, g, H of every moving vertex at the current positions
 // (the f64 gradient check of src/gpu_vbd.rs:305-379, probe of vbd.wgsl:142-147).
-__global__ void k_local_blocks(SweepView s, double* energy, double* grad, double* hess) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < s.n; v += gridDim.x * blockDim.x) {
+template <int G>
+__global__ void __launch_bounds__(128) k_local_blocks(SweepView s, double* energy, double* grad, double* hess) {
+    __shared__ double near_s[128 / G * Near<G>::kDoubles];
+    const uint32_t lane = threadIdx.x & (G - 1);
+    const unsigned mask = ((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1));
+    for (uint32_t v = (blockIdx.x * 128 + threadIdx.x) / G; v < s.n; v += gridDim.x * 128 / G) {
         d3 x = ld3(s.x, v);
+        Near<G> T;
+        T.head(s, v);
+        const typename Near<G>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
         d3 g = mk(0, 0, 0);
         Sym H;
         sym_zero(H);
-        double e = local_part<true, 1>(s, v, x, 0, g, H);
+        double e = group_sum<G>(local_part<true, G>(s, T, f, x, lane, g, H), mask);
+        g = mk(group_sum<G>(g.x, mask), group_sum<G>(g.y, mask), group_sum<G>(g.z, mask));
+        for (int k = 0; k < 6; ++k) H.a[k] = group_sum<G>(H.a[k], mask);
+        if (lane != 0) continue;
         double m = s.inertia ? s.inertia[v] : 0.0;
         d3 y = s.target ? ld3(s.target, v) : x;
         d3 xy = x - y;
@@ -242,7 +255,72 @@ __global__ void k_local_blocks(SweepView s, double* energy, double* grad, double
 }
 
 void launch_local_blocks(const SweepView& s, double* energy, double* grad, double* hess, cudaStream_t st) {
-    k_local_blocks<<<grid_for(s.n, 128), 128, 0, st>>>(s, energy, grad, hess);
+    k_local_blocks<8><<<grid_for(8 * (size_t)s.n, 128), 128, 0, st>>>(s, energy, grad, hess);
+}
+
+// Heads in colour order: what a solve needs of its vertex before it can ask for
+// anything else, side by side for the groups of a sweep.
+__global__ void k_color_heads(SweepView s, const uint32_t* order, uint4* heads) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += gridDim.x * blockDim.x) {
+        const uint32_t v = order[i];
+        const uint4 a = s.vt.head[2 * (size_t)v], b = s.vt.head[2 * (size_t)v + 1];
+        heads[3 * (size_t)i] = make_uint4(v, a.x, a.y, a.z);
+        heads[3 * (size_t)i + 1] = make_uint4(s.pinned[v] ? kPinnedHead : a.w, b.x, b.y, b.z);
+        heads[3 * (size_t)i + 2] = make_uint4(b.w, s.contacts.inc_off[v], s.contacts.inc_off[v + 1], 0u);
+    }
+}
+
+void launch_color_heads(const SweepView& s, const uint32_t* order, uint4* heads, cudaStream_t st) {
+    if (s.n == 0) return;
+    k_color_heads<<<grid_for(s.n, 256), 256, 0, st>>>(s, order, heads);
+    CC_CUDA(cudaGetLastError());
+}
+
+// Records of VertexTerms from the per-element data, one thread per vertex.
+__global__ void k_vertex_terms(SweepView s, unsigned long long* tri, double4* tri_b, double4* tri_k,
+                               ulonglong2* hinge) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < s.n; v += gridDim.x * blockDim.x) {
+        const uint4 a = s.vt.head[2 * (size_t)v], b = s.vt.head[2 * (size_t)v + 1];
+        auto place = [&](uint32_t id) {  // in the ascending neighbour list
+            uint32_t lo = 0, hi = a.y;
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (s.vt.nb[a.x + mid] < id) lo = mid + 1;
+                else hi = mid;
+            }
+            return (unsigned long long)lo;
+        };
+        const uint32_t* inc = s.inc + s.inc_off[v];
+        for (uint32_t i = 0; i < a.w; ++i) {
+            const uint32_t t = inc[i] & 0x0fffffffu, slot = (inc[i] >> 28) & 3u;
+            const int4 tv = s.tri_v[t];
+            const double4 c = s.tri_coef[t];
+            const MatParams M = s.mats[tv.w];
+            const double A = s.tri_area[t];
+            // w and v are differences: the weights of the three vertices add up to zero
+            const double w0 = -(c.x + c.y), v0 = -(c.z + c.w);
+            const uint32_t j = (uint32_t)(slot == 0 ? tv.y : tv.x), k = (uint32_t)(slot == 2 ? tv.y : tv.z);
+            tri[a.z + i] = place(j) | place(k) << 21 | (unsigned long long)(uint32_t)tv.w << 42;
+            tri_b[a.z + i] = make_double4(slot == 0 ? c.x : w0, slot == 2 ? c.x : c.y, slot == 0 ? c.z : v0,
+                                          slot == 2 ? c.z : c.w);
+            tri_k[a.z + i] = make_double4(A * M.warp, A * M.weft, A * M.shear, M.c);
+        }
+        // the hinges of which v is an end of the shared edge (slots 0, 1), then those of which it is a wing
+        uint32_t ends = b.x, wings = b.x + b.y;
+        for (uint32_t i = 0; i < b.y + b.z; ++i) {
+            const uint32_t ent = inc[a.w + i], h = ent & 0x0fffffffu, slot = (ent >> 28) & 3u;
+            const uint3 q = hinge_points(s.hinge_v[h], slot);
+            hinge[slot < 2 ? ends++ : wings++] = make_ulonglong2(place(q.x) | place(q.y) << 21 | place(q.z) << 42,
+                                             (unsigned long long)__double_as_longlong(s.hinge_k[h]));
+        }
+    }
+}
+
+void launch_vertex_terms(const SweepView& s, unsigned long long* tri, double4* tri_b, double4* tri_k,
+                         ulonglong2* hinge, cudaStream_t st) {
+    if (s.n == 0) return;
+    k_vertex_terms<<<grid_for(s.n, 128), 128, 0, st>>>(s, tri, tri_b, tri_k, hinge);
+    CC_CUDA(cudaGetLastError());
 }
 
 // ------------------------------------------ step objective and its gradient
@@ -256,6 +334,7 @@ void launch_local_blocks(const SweepView& s, double* energy, double* grad, doubl
 template <int G>
 __global__ void __launch_bounds__(128) k_grad_sq(SweepView s, double* out, const unsigned* skip_at, uint32_t iteration,
                                                  int project) {
+    __shared__ double near_s[128 / G * Near<G>::kDoubles];
     if (skip_at && *skip_at <= iteration) return;
     uint32_t t = blockIdx.x * 128 + threadIdx.x;
     uint32_t v = t / G;
@@ -270,7 +349,10 @@ __global__ void __launch_bounds__(128) k_grad_sq(SweepView s, double* out, const
     d3 g = mk(0, 0, 0);
     Sym H;
     sym_zero(H);
-    local_part<true, G, false>(s, v, x, lane, g, H);  // gradient only
+    Near<G> T;
+    T.head(s, v);
+    const typename Near<G>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
+    local_part<true, G, false>(s, T, f, x, lane, g, H);  // gradient only
     if (G > 1) {
         g.x = group_sum<G>(g.x, mask);
         g.y = group_sum<G>(g.y, mask);
@@ -319,17 +401,14 @@ __global__ void k_term_energy(SweepView s, ObjectiveCounts c, double* out) {
                 e = 0.5 * s.inertia[k] * dot(d, d);
             }
         } else if ((k -= s.n) < c.triangles) {
-            uint32_t v = (uint32_t)s.tri_v[k].x;
-            e = membrane_term<false>(s, (uint32_t)k, 0, ld3(s.x, v), g, H);
+            e = membrane_energy(s, (uint32_t)k);
         } else if ((k -= c.triangles) < c.hinges) {
-            uint32_t v = s.hinge_v[k].x;
-            e = bending_term<false>(s, (uint32_t)k, 0, ld3(s.x, v), g, H);
+            e = bending_energy(s, (uint32_t)k);
         } else if ((k -= c.hinges) < c.stitches) {
             uint32_t v = s.st_v[s.st_off[k]];
             e = stitch_term<false>(s, (uint32_t)k, v, ld3(s.x, v), g, H);
         } else if ((k -= c.stitches) < c.contacts) {
-            uint32_t v = s.contacts.verts[k].x;
-            e = contact_term<false>(s, (uint32_t)k, v, ld3(s.x, v), g, H);
+            e = contact_energy(s, (uint32_t)k);
         } else if (s.grab.active) {
             uint32_t v = s.grab.v[0];
             e = grab_term<false>(s, v, ld3(s.x, v), g, H);

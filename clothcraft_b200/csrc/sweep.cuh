@@ -25,6 +25,25 @@ struct GrabDev {
     double k;
 };
 
+// A vertex's elastic terms as the local solves read them (k_vertex_terms): one
+// record per (vertex, term), a vertex's records side by side, with the term's
+// other vertices named by their place in the vertex's neighbour list and the
+// element data turned to the vertex's point of view. A solve then reads one head,
+// one list of ids and one position per neighbour, and coalesced records, where
+// per-element data took head -> entry -> element -> positions, with each
+// neighbour's position read four times.
+struct VertexTerms {
+    const uint4* head;  // [2n] {first neighbour, neighbours, first triangle record, triangles},
+                        //      {first hinge record, edge-end hinges, wing hinges, stitches}
+    const uint32_t* nb;                // neighbour ids, ascending (the material graph)
+    const unsigned long long* tri;     // neighbours j | k << 21 | material << 42
+    const double4* tri_b;              // fibre vectors w = dj b.x + dk b.y, v = dj b.z + dk b.w (d = neighbour - vertex)
+    const double4* tri_k;              // area * (warp, weft, shear), compression ratio
+    const ulonglong2* hinge;           // neighbours a | b << 21 | c << 42 (hinge_points), bits of K
+};
+
+constexpr uint32_t kPinnedHead = ~0u;
+
 struct SweepView {
     uint32_t n;                 // moving vertices
     double4* x;                 // [n_all] positions (moving part written)
@@ -45,6 +64,11 @@ struct SweepView {
     const uint32_t* st_v;
     const double* st_w;
     const double* st_k;
+    VertexTerms vt;
+    // [3 per vertex of the launch] the colour's vertices in order (k_color_heads): {vertex, first neighbour,
+    // neighbours, first triangle record}, {triangles or kPinnedHead, first hinge record, edge-end hinges, wing
+    // hinges}, {stitches, first contact entry, end of the contact entries, 0}
+    const uint4* heads;
     ContactsView contacts;
     double contact_r, contact_k;
     GrabDev grab;
@@ -104,9 +128,15 @@ inline SweepVariant decode_variant(int v) {
 // valid variants of the FP64 (fp32 = false) and FP32-assembly sweeps
 bool sweep_variant_valid(int v, bool fp32);
 
+// Fills the records of vt (buffers sized by the heads) from the per-element
+// data of s; once per solver.
+void launch_vertex_terms(const SweepView& s, unsigned long long* tri, double4* tri_b, double4* tri_k,
+                         ulonglong2* hinge, cudaStream_t st);
 // launch helpers (sweep.cu); grid_cap > 0 limits the grid (persistent variants)
-void launch_sweep(const SweepView& s, const uint32_t* order, uint32_t count, int variant, cudaStream_t st,
-                  unsigned grid_cap = 0);
+// (s.heads: the colour's)
+void launch_sweep(const SweepView& s, uint32_t count, int variant, cudaStream_t st, unsigned grid_cap = 0);
+// heads of all vertices in `order`; after every colouring
+void launch_color_heads(const SweepView& s, const uint32_t* order, uint4* heads, cudaStream_t st);
 // FP32 element assembly (sweep32.cu); lanes 4, 8, 16 or 32
 void launch_sweep32(const SweepView& s, const uint32_t* order, uint32_t count, int variant, cudaStream_t st,
                     unsigned grid_cap = 0);

@@ -25,7 +25,7 @@
 // memory in each trial.
 #include <atomic>
 
-#include "sweep_terms.cuh"
+#include "contact_jet.cuh"
 
 namespace cc {
 
@@ -361,7 +361,7 @@ __device__ __forceinline__ void solve_vertex32(const SweepView& s, uint32_t v, u
     const bool grab_here = lane == 0 && s.grab.active && (s.grab.v[0] == v || s.grab.v[1] == v || s.grab.v[2] == v);
     const bool lane64 = (mid.y + lane < b1) || (c0 + lane < c1) || grab_here;
     for (uint32_t k = mid.y + lane; k < b1; k += G) e64 += stitch_term<true>(s, s.inc[k] & 0x0fffffffu, v, x, g64, H64);
-    for (uint32_t k = c0 + lane; k < c1; k += G) e64 += contact_term<true>(s, s.contacts.inc[k], v, x, g64, H64);
+    for (uint32_t k = c0 + lane; k < c1; k += G) e64 += jet::contact_term<true>(s, s.contacts.inc[k], v, x, g64, H64);
     if (grab_here) e64 += grab_term<true>(s, v, x, g64, H64);
     const bool any64 = G > 1 ? __any_sync(mask, lane64) : lane64;
     if (G > 1) {
@@ -462,7 +462,7 @@ __device__ __forceinline__ void solve_vertex32(const SweepView& s, uint32_t v, u
             double e1 = 0.0;
             for (uint32_t k = mid.y + lane; k < b1; k += G)
                 e1 += stitch_term<false>(s, s.inc[k] & 0x0fffffffu, v, cand, gd, Hd);
-            for (uint32_t k = c0 + lane; k < c1; k += G) e1 += contact_term<false>(s, s.contacts.inc[k], v, cand, gd, Hd);
+            for (uint32_t k = c0 + lane; k < c1; k += G) e1 += jet::contact_term<false>(s, s.contacts.inc[k], v, cand, gd, Hd);
             if (grab_here) e1 += grab_term<false>(s, v, cand, gd, Hd);
             de += e1 - e64;
         }

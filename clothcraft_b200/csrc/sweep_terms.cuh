@@ -1,7 +1,7 @@
 // Device-side terms of the VBD local solve shared by the FP64 sweep
 // (sweep.cu) and the FP32-assembly sweep (sweep32.cu): 3x3 symmetric blocks,
-// the FP64 membrane and bending terms with exact derivatives, stitches, the
-// grab, and the OGC contact energy with its forward-mode (Jet3) derivatives.
+// the FP64 membrane and bending terms, stitches, the grab and the OGC contact
+// energy, all with exact derivatives in closed form.
 #pragma once
 #include "sweep.cuh"
 
@@ -69,110 +69,119 @@ __device__ __forceinline__ d3 pos(const SweepView& s, uint32_t i, uint32_t v, d3
     return i == v ? p : ld3(s.x, i);
 }
 
-// membrane (src/energy.rs:17-29) of triangle t with vertex slot `slot` at p.
-// D: derivatives; HS: also the Hessian (a gradient-only evaluation skips it)
+// membrane (src/energy.rs:17-29) with one vertex at p; dj, dk: the other two
+// vertices less p; b, k as VertexTerms has them. D: derivatives; HS: also the
+// Hessian (a gradient-only evaluation skips it)
 template <bool D, bool HS = D>
-__device__ __forceinline__ double membrane_rec(const SweepView& s, int4 tv, double4 cf, double A, uint32_t slot, d3 p,
-                                               d3& g, Sym& H) {
-    MatParams M = s.mats[tv.w];
-    d3 x0 = slot == 0 ? p : ld3(s.x, (uint32_t)tv.x);
-    d3 x1 = slot == 1 ? p : ld3(s.x, (uint32_t)tv.y);
-    d3 x2 = slot == 2 ? p : ld3(s.x, (uint32_t)tv.z);
-    d3 ds0 = x1 - x0, ds1 = x2 - x0;
-    d3 w = ds0 * cf.x + ds1 * cf.y;
-    d3 v = ds0 * cf.z + ds1 * cf.w;
-    double ew = (dot(w, w) - 1.0) * 0.5;
-    double ev = (dot(v, v) - 1.0) * 0.5;
-    double sh = dot(w, v);
-    if (!D) return A * (axial1(ew, M.warp, M.c, M.delta) + axial1(ev, M.weft, M.c, M.delta) + 0.5 * M.shear * sh * sh);
+__device__ __forceinline__ double membrane(const SweepView& s, double4 b, double4 k, uint32_t mat, d3 dj, d3 dk, d3& g,
+                                           Sym& H) {
+    const d3 w = dj * b.x + dk * b.y, v = dj * b.z + dk * b.w;
+    const double ew = (dot(w, w) - 1.0) * 0.5, ev = (dot(v, v) - 1.0) * 0.5, sh = dot(w, v);
+    const double delta = k.w == 1.0 ? 0.0 : s.mats[mat].delta;  // unused by the pure quadratic law
+    if (!D) return axial1(ew, k.x, k.w, delta) + axial1(ev, k.y, k.w, delta) + 0.5 * k.z * sh * sh;
     double fw, fw1, fw2, fv, fv1, fv2;
-    axial3(ew, M.warp, M.c, M.delta, fw, fw1, fw2);
-    axial3(ev, M.weft, M.c, M.delta, fv, fv1, fv2);
-    double aw = slot == 0 ? -(cf.x + cf.y) : (slot == 1 ? cf.x : cf.y);
-    double av = slot == 0 ? -(cf.z + cf.w) : (slot == 1 ? cf.z : cf.w);
-    d3 q = v * aw + w * av;
-    g = g + (w * (fw1 * aw) + v * (fv1 * av) + q * (M.shear * sh)) * A;
-    if (!HS) return A * (fw + fv + 0.5 * M.shear * sh * sh);
-    sym_add_outer(H, w, A * fw2 * aw * aw);
-    sym_add_outer(H, v, A * fv2 * av * av);
-    sym_add_outer(H, q, A * M.shear);
-    sym_add_diag(H, A * (fw1 * aw * aw + fv1 * av * av + 2.0 * M.shear * sh * aw * av));
-    return A * (fw + fv + 0.5 * M.shear * sh * sh);
+    axial3(ew, k.x, k.w, delta, fw, fw1, fw2);
+    axial3(ev, k.y, k.w, delta, fv, fv1, fv2);
+    const double aw = -(b.x + b.y), av = -(b.z + b.w);  // the rates of w and v in p
+    const d3 q = v * aw + w * av;
+    g = g + w * (fw1 * aw) + v * (fv1 * av) + q * (k.z * sh);
+    if (HS) {
+        sym_add_outer(H, w, fw2 * aw * aw);
+        sym_add_outer(H, v, fv2 * av * av);
+        sym_add_outer(H, q, k.z);
+        sym_add_diag(H, fw1 * aw * aw + fv1 * av * av + 2.0 * k.z * sh * aw * av);
+    }
+    return fw + fv + 0.5 * k.z * sh * sh;
 }
 
+// energy of triangle t alone
+__device__ __forceinline__ double membrane_energy(const SweepView& s, uint32_t t) {
+    const int4 tv = s.tri_v[t];
+    const double4 c = s.tri_coef[t];
+    const double A = s.tri_area[t];
+    const MatParams M = s.mats[tv.w];
+    const d3 p = ld3(s.x, (uint32_t)tv.x);
+    d3 g;
+    Sym H;
+    return membrane<false>(s, c, make_double4(A * M.warp, A * M.weft, A * M.shear, M.c), (uint32_t)tv.w,
+                           ld3(s.x, (uint32_t)tv.y) - p, ld3(s.x, (uint32_t)tv.z) - p, g, H);
+}
+
+// bending (src/energy.rs:31-46): K |h1 - h2|^2 of a hinge's unit normals, which
+// is 2K (1 - cos t) of the dihedral angle t. With sin t = S and cos t = h1.h2
+// the derivatives in one vertex are 2K S grad t and 2K (cos t grad t grad t^T +
+// S Hess t). A vertex is either an end of the shared edge or a wing (the corner
+// of one triangle opposite the edge), and the two have their own closed forms
+// (bending_edge, bending_wing); a hinge's corners in the order that the form
+// needs are hinge_points. Generic second derivatives of both normals (skew
+// matrices and projections) took ~250 FP64 operations for either role; these
+// take ~70 (wing) and ~130 (edge).
+
+// Corners of hinge (x0 x1 the edge, x2 and x3 the wings) as seen from slot:
+// edge ends: {other end, wing A, wing B} with nA = (o - A) x (o - p) and
+// nB = (o - p) x (o - B); wings: {edge, edge, other wing} with n1 = e x (p - x0).
+// Renaming (x0, x1, x2, x3) -> (x1, x0, x3, x2) keeps both normals, so slots 1
+// and 3 are slots 0 and 2 of the renamed hinge.
+__device__ __forceinline__ uint3 hinge_points(uint4 hv, uint32_t slot) {
+    switch (slot) {
+        case 0: return make_uint3(hv.y, hv.z, hv.w);
+        case 1: return make_uint3(hv.x, hv.w, hv.z);
+        case 2: return make_uint3(hv.x, hv.y, hv.w);
+        default: return make_uint3(hv.y, hv.x, hv.z);
+    }
+}
+
+// An end p of the shared edge. grad t = -(fA + fB) with f = (a.e) n / (|e| |n|^2),
+// a from the wing to the other end and e = o - p; Hess t is the symmetric part of
+// sum n (df/de)^T.
 template <bool D, bool HS = D>
-__device__ __forceinline__ double membrane_term(const SweepView& s, uint32_t t, uint32_t slot, d3 p, d3& g, Sym& H) {
-    return membrane_rec<D, HS>(s, s.tri_v[t], s.tri_coef[t], s.tri_area[t], slot, p, g, H);
-}
-
-// P_k [a]x / l as three columns: P(a x e_j)/l, P y = y - h (h.y)
-__device__ __forceinline__ void proj_skew_cols(d3 a, d3 h, double inv_l, double sign, d3& c0, d3& c1, d3& c2) {
-    d3 e0 = mk(0.0, a.z, -a.y), e1 = mk(-a.z, 0.0, a.x), e2 = mk(a.y, -a.x, 0.0);
-    double f = sign * inv_l;
-    c0 = c0 + (e0 - h * dot(h, e0)) * f;
-    c1 = c1 + (e1 - h * dot(h, e1)) * f;
-    c2 = c2 + (e2 - h * dot(h, e2)) * f;
-}
-
-// [a]x^T M [a]x for M = -(1/l^2)[d h^T + h d^T + (d.h)(I - 3 h h^T)]
-__device__ __forceinline__ void add_curvature(Sym& Hm, d3 a, d3 h, d3 d, double inv_l2, double sign) {
-    d3 da = cross(d, a), ha = cross(h, a);
-    double dh = dot(d, h);
-    double sc = -inv_l2 * sign;
-    sym_add_outer2(Hm, da, ha, sc);
-    double aa = dot(a, a);
-    sym_add_diag(Hm, sc * dh * aa);
-    sym_add_outer(Hm, a, -sc * dh);
-    sym_add_outer(Hm, ha, -3.0 * sc * dh);
-}
-
-// bending (src/energy.rs:31-46) of hinge h with vertex slot `slot` at p.
-// n1 = e x u, n2 = w x e are affine in one vertex: dn_k/dp = [a_k]x.
-template <bool D, bool HS = D>
-__device__ __forceinline__ double bending_rec(const SweepView& s, uint4 hv, double K, uint32_t slot, d3 p, d3& g,
-                                              Sym& H) {
-    d3 x0 = slot == 0 ? p : ld3(s.x, hv.x);
-    d3 x1 = slot == 1 ? p : ld3(s.x, hv.y);
-    d3 x2 = slot == 2 ? p : ld3(s.x, hv.z);
-    d3 x3 = slot == 3 ? p : ld3(s.x, hv.w);
-    d3 e = x1 - x0, u = x2 - x0, w = x3 - x0;
-    d3 n1 = cross(e, u);
-    d3 n2 = cross(w, e);
-    double il1 = rsqrt(dot(n1, n1));
-    double il2 = rsqrt(dot(n2, n2));
-    d3 h1 = n1 * il1, h2 = n2 * il2;
-    d3 d = h1 - h2;
-    double energy = K * dot(d, d);
+__device__ __forceinline__ double bending_edge(double K, d3 o, d3 xa, d3 xb, d3 p, d3& g, Sym& H) {
+    const d3 e = o - p, a = o - xa, b = o - xb;
+    const d3 na = cross(a, e), nb = cross(e, b);
+    const double la = rsqrt(dot(na, na)), lb = rsqrt(dot(nb, nb));
+    const d3 ha = na * la, hb = nb * lb;
+    const d3 d = ha - hb;
+    const double energy = K * dot(d, d);
     if (!D) return energy;
-    d3 a1 = slot == 0 ? u - e : (slot == 1 ? -u : (slot == 2 ? e : mk(0, 0, 0)));
-    d3 a2 = slot == 0 ? e - w : (slot == 1 ? w : (slot == 3 ? -e : mk(0, 0, 0)));
-    // gradient 2K J^T d with J^T d = sum_k s_k ((P_k d) x a_k) / l_k
-    d3 pd1 = d - h1 * dot(h1, d), pd2 = d - h2 * dot(h2, d);
-    d3 jtd = cross(pd1, a1) * il1 - cross(pd2, a2) * il2;
-    g = g + jtd * (2.0 * K);
+    const double ie = 1.0 / dot(e, e);
+    const double ae = dot(a, e), be = dot(b, e);
+    const d3 f = ha * (ae * la) + hb * (be * lb);            // |e| (fA + fB)
+    const double q = 2.0 * K * ie * dot(e, cross(hb, ha));  // 2K S / |e|
+    g = g - f * q;
     if (!HS) return energy;
-    // Hessian 2K [J^T J + A1^T M1 A1 - A2^T M2 A2]
-    d3 c0 = mk(0, 0, 0), c1 = mk(0, 0, 0), c2 = mk(0, 0, 0);
-    proj_skew_cols(a1, h1, il1, 1.0, c0, c1, c2);
-    proj_skew_cols(a2, h2, il2, -1.0, c0, c1, c2);
-    Sym Hm;
-    Hm.a[0] = dot(c0, c0);
-    Hm.a[1] = dot(c0, c1);
-    Hm.a[2] = dot(c0, c2);
-    Hm.a[3] = dot(c1, c1);
-    Hm.a[4] = dot(c1, c2);
-    Hm.a[5] = dot(c2, c2);
-    add_curvature(Hm, a1, h1, d, il1 * il1, 1.0);
-    add_curvature(Hm, a2, h2, d, il2 * il2, -1.0);
-    double f = 2.0 * K;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) H.a[k] += f * Hm.a[k];
+    sym_add_outer(H, f, 2.0 * K * ie * dot(ha, hb));
+    const d3 va = a - e * (ae * ie) - cross(ha, a) * (2.0 * ae * la);
+    const d3 vb = b - e * (be * ie) - cross(b, hb) * (2.0 * be * lb);
+    sym_add_outer2(H, ha, va, 0.5 * q * la);
+    sym_add_outer2(H, hb, vb, 0.5 * q * lb);
     return energy;
 }
 
+// A wing p: only its own normal moves, turning about the edge e with p:
+// grad t = h |e| / |n|, Hess t = -(|e|^2 / |n|^2) (t h^T + h t^T), t = h x e / |e|.
 template <bool D, bool HS = D>
-__device__ __forceinline__ double bending_term(const SweepView& s, uint32_t hi, uint32_t slot, d3 p, d3& g, Sym& H) {
-    return bending_rec<D, HS>(s, s.hinge_v[hi], s.hinge_k[hi], slot, p, g, H);
+__device__ __forceinline__ double bending_wing(double K, d3 x0, d3 x1, d3 x3, d3 p, d3& g, Sym& H) {
+    const d3 e = x1 - x0;
+    const d3 n1 = cross(e, p - x0), n2 = cross(x3 - x0, e);
+    const double l1 = rsqrt(dot(n1, n1)), l2 = rsqrt(dot(n2, n2));
+    const d3 h1 = n1 * l1, h2 = n2 * l2;
+    const d3 d = h1 - h2;
+    const double energy = K * dot(d, d);
+    if (!D) return energy;
+    const double q = 2.0 * K * l1 * dot(e, cross(h2, h1));  // 2K S |e| / |n1|
+    g = g + h1 * q;
+    if (!HS) return energy;
+    sym_add_outer(H, h1, 2.0 * K * l1 * l1 * dot(h1, h2) * dot(e, e));
+    sym_add_outer2(H, cross(h1, e), h1, -q * l1);
+    return energy;
+}
+
+// energy of hinge h alone
+__device__ __forceinline__ double bending_energy(const SweepView& s, uint32_t h) {
+    const uint4 v = s.hinge_v[h];
+    d3 g;
+    Sym H;
+    return bending_wing<false>(s.hinge_k[h], ld3(s.x, v.x), ld3(s.x, v.y), ld3(s.x, v.w), ld3(s.x, v.z), g, H);
 }
 
 // stitch 0.5 k |sum w_j x_j|^2 (src/vbd.rs:217-227)
@@ -194,289 +203,134 @@ __device__ __forceinline__ double stitch_term(const SweepView& s, uint32_t st, u
     return 0.5 * K * dot(d, d);
 }
 
-// ----------------------------------------------- contact: forward-mode AD
-// Jet3 with a symmetric Hessian: the second-order chain rules of
-// src/math.rs:46-122, restricted to one vertex's three coordinates.
-struct J3 {
-    double v;
-    double g0, g1, g2;
-    double h00, h01, h02, h11, h12, h22;
-};
-__device__ __forceinline__ J3 jc(double v) { return {v, 0, 0, 0, 0, 0, 0, 0, 0, 0}; }
-__device__ __forceinline__ J3 operator+(const J3& a, const J3& b) {
-    return {a.v + b.v,     a.g0 + b.g0,   a.g1 + b.g1,   a.g2 + b.g2,   a.h00 + b.h00,
-            a.h01 + b.h01, a.h02 + b.h02, a.h11 + b.h11, a.h12 + b.h12, a.h22 + b.h22};
-}
-__device__ __forceinline__ J3 operator-(const J3& a, const J3& b) {
-    return {a.v - b.v,     a.g0 - b.g0,   a.g1 - b.g1,   a.g2 - b.g2,   a.h00 - b.h00,
-            a.h01 - b.h01, a.h02 - b.h02, a.h11 - b.h11, a.h12 - b.h12, a.h22 - b.h22};
-}
-__device__ __forceinline__ J3 operator-(const J3& a) {
-    return {-a.v, -a.g0, -a.g1, -a.g2, -a.h00, -a.h01, -a.h02, -a.h11, -a.h12, -a.h22};
-}
-__device__ __forceinline__ J3 operator*(const J3& a, const J3& b) {
-    J3 r;
-    r.v = a.v * b.v;
-    r.g0 = a.g0 * b.v + a.v * b.g0;
-    r.g1 = a.g1 * b.v + a.v * b.g1;
-    r.g2 = a.g2 * b.v + a.v * b.g2;
-    r.h00 = a.h00 * b.v + a.v * b.h00 + 2.0 * a.g0 * b.g0;
-    r.h01 = a.h01 * b.v + a.v * b.h01 + a.g0 * b.g1 + b.g0 * a.g1;
-    r.h02 = a.h02 * b.v + a.v * b.h02 + a.g0 * b.g2 + b.g0 * a.g2;
-    r.h11 = a.h11 * b.v + a.v * b.h11 + 2.0 * a.g1 * b.g1;
-    r.h12 = a.h12 * b.v + a.v * b.h12 + a.g1 * b.g2 + b.g1 * a.g2;
-    r.h22 = a.h22 * b.v + a.v * b.h22 + 2.0 * a.g2 * b.g2;
-    return r;
-}
-__device__ __forceinline__ J3 chain(const J3& a, double value, double f1, double f2) {
-    J3 r;
-    r.v = value;
-    r.g0 = f1 * a.g0;
-    r.g1 = f1 * a.g1;
-    r.g2 = f1 * a.g2;
-    r.h00 = f1 * a.h00 + f2 * a.g0 * a.g0;
-    r.h01 = f1 * a.h01 + f2 * a.g0 * a.g1;
-    r.h02 = f1 * a.h02 + f2 * a.g0 * a.g2;
-    r.h11 = f1 * a.h11 + f2 * a.g1 * a.g1;
-    r.h12 = f1 * a.h12 + f2 * a.g1 * a.g2;
-    r.h22 = f1 * a.h22 + f2 * a.g2 * a.g2;
-    return r;
-}
-__device__ __forceinline__ J3 operator/(const J3& a, const J3& b) {
-    return a * chain(b, 1.0 / b.v, -1.0 / (b.v * b.v), 2.0 / (b.v * b.v * b.v));
-}
-__device__ __forceinline__ J3 ssqrt(const J3& a) {
-    double r = sqrt(a.v);
-    return chain(a, r, 0.5 / r, -0.25 / (r * r * r));
-}
-__device__ __forceinline__ J3 sln(const J3& a) { return chain(a, log(a.v), 1.0 / a.v, -1.0 / (a.v * a.v)); }
-__device__ __forceinline__ double ssqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ double sln(double x) { return log(x); }
-__device__ __forceinline__ double sval(double x) { return x; }
-__device__ __forceinline__ double sval(const J3& x) { return x.v; }
-template <class S>
-__device__ __forceinline__ S scst(double v);
-template <>
-__device__ __forceinline__ double scst<double>(double v) {
-    return v;
-}
-template <>
-__device__ __forceinline__ J3 scst<J3>(double v) {
-    return jc(v);
+// ---------------------------------------------------------------- contact
+// Contact::energy (src/ogc/potential.rs:39-65): an activation of the distance d
+// of two features, for edge pairs times a mollifier of |n|^2. One vertex p of
+// the contact moves; its derivatives are closed forms (second-order forward
+// differentiation of the same expressions, ten components a value, took ~8 times
+// the operations). The vertex's part in the contact is c.w (ContactRole) and the
+// other points are c.x, c.y, c.z. For the last three roles d = |w.n| with
+// n = g x f / |g x f|.
+
+// activation (src/ogc/potential.rs:8-22) with its derivatives, d < r
+__device__ __forceinline__ double activation(double d, double r, double k, double& f1, double& f2) {
+    const double tau = 0.5 * r;
+    if (d >= tau) {
+        f1 = -k * (r - d);
+        f2 = k;
+        return 0.5 * k * (r - d) * (r - d);
+    }
+    f1 = f2 = 0.0;
+    if (d <= 0.0) return __longlong_as_double(0x7ff0000000000000ll);
+    const double kt = k * tau * tau, id = 1.0 / d;
+    f1 = -kt * id;
+    f2 = kt * id * id;
+    return 0.5 * kt - kt * log(d / tau);
 }
 
-template <class S>
-struct V {
-    S x, y, z;
-};
-template <class S>
-__device__ __forceinline__ V<S> vsub(const V<S>& a, const V<S>& b) {
-    return {a.x - b.x, a.y - b.y, a.z - b.z};
-}
-template <class S>
-__device__ __forceinline__ S vdot(const V<S>& a, const V<S>& b) {
-    return a.x * b.x + a.y * b.y + a.z * b.z;
-}
-template <class S>
-__device__ __forceinline__ V<S> vcross(const V<S>& a, const V<S>& b) {
-    return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+// Energy of the term with p at the moving vertex, and its gradient and Hessian.
+// A term at d >= r adds nothing.
+template <bool D, bool HS = D>
+__device__ __forceinline__ double contact_rec(const SweepView& s, uint4 c, double eps, d3 p, d3& g, Sym& H) {
+    const double r = s.contact_r, k = s.contact_k;
+    double f1, f2;
+    if (c.w <= ON_LINE) {
+        d3 n;
+        double d, t = -1.0, iu = 0.0;  // the gradient of d is -t n
+        d3 u = mk(0, 0, 0);
+        const d3 a = ld3(s.x, c.x);
+        if (c.w == POINT) {
+            n = p - a;
+        } else {
+            const d3 b = ld3(s.x, c.y);
+            const d3 w = (c.w == FROM_LINE ? p : b) - a;
+            u = (c.w == FROM_LINE ? b : p) - a;
+            iu = 1.0 / dot(u, u);
+            const double q = dot(w, u) * iu;
+            if (c.w == ON_LINE) t = q;
+            n = w - u * q;
+        }
+        d = sqrt(dot(n, n));
+        if (d >= r) return 0.0;
+        const double e = activation(d, r, k, f1, f2);
+        if (!D || d <= 0.0) return e;
+        const double id = 1.0 / d;
+        n = n * id;
+        g = g - n * (f1 * t);
+        if (!HS) return e;
+        // f2 t^2 n n^T + f1 Hess d, Hess d = (t^2 / d)(I - n n^T - u u^T / u^2)
+        //   [ON_LINE: - (d / u^2) n n^T + (t / u^2)(n u^T + u n^T)]
+        const double h = f1 * t * t * id;
+        const bool end = c.w == ON_LINE;
+        sym_add_diag(H, h);
+        sym_add_outer(H, n, f2 * t * t - h - (end ? f1 * d * iu : 0.0));
+        if (c.w != POINT) sym_add_outer(H, u, -h * iu);
+        if (end) sym_add_outer2(H, n, u, f1 * t * iu);
+        return e;
+    }
+    const d3 a = ld3(s.x, c.x), b = ld3(s.x, c.y), o = ld3(s.x, c.z);
+    const bool edges = c.w == EDGES;
+    const d3 f = edges ? o - b : b - a;
+    const d3 e1 = c.w == FROM_PLANE ? o - a : p - a;
+    const d3 w = c.w == FROM_PLANE ? p - a : (edges ? a - b : o - a);
+    const d3 N = cross(e1, f);
+    const double NN = dot(N, N);
+    if (edges && NN < 1e-30) return 0.0;
+    const double il = rsqrt(NN);
+    const double h = dot(w, N) * il, d = fabs(h);
+    if (d >= r) return 0.0;
+    double e = activation(d, r, k, f1, f2);
+    double psi = 1.0, psi1 = 0.0;
+    const double qm = edges ? NN / eps : 1.0;
+    if (qm < 1.0) {
+        psi = qm * (2.0 - qm);
+        psi1 = 2.0 - 2.0 * qm;
+    }
+    const double energy = e * psi;
+    if (!D) return energy;
+    if (d <= 0.0) {
+        // touching features have infinite energy and no direction; mollified, no finite derivative either
+        if (qm < 1.0) g.x = __longlong_as_double(0x7ff8000000000000ll);
+        return energy;
+    }
+    const double sg = h < 0.0 ? -1.0 : 1.0;
+    const d3 n = N * il;
+    // n turns about f as p leaves the plane: grad h = -l n, Hess h = -h |m|^2 n n^T + l (m n^T + n m^T),
+    // m = f x n / |N|, l = w.m; from the plane's point grad h = n
+    const bool from = c.w == FROM_PLANE;
+    const d3 m = cross(f, n) * il;
+    const double l = from ? -1.0 : dot(w, m);
+    d3 gh = n * (-l * sg * f1);  // gradient of the activation
+    if (HS) {
+        double on = psi * f2 * l * l;
+        if (!from) {
+            on -= psi * f1 * d * dot(m, m);
+            sym_add_outer2(H, m, n, psi * f1 * sg * l);
+        }
+        sym_add_outer(H, n, on);
+    }
+    if (qm < 1.0) {
+        // q = |N|^2 / eps: grad q = 2 f x N / eps, Hess q = 2 (f^2 I - f f^T) / eps
+        const d3 gq = cross(f, N) * (2.0 / eps);
+        if (HS) {
+            sym_add_outer2(H, gh, gq, psi1);
+            sym_add_outer(H, gq, -2.0 * e);
+            const double hq = e * psi1 * 2.0 / eps;
+            sym_add_diag(H, hq * dot(f, f));
+            sym_add_outer(H, f, -hq);
+        }
+        gh = gh * psi + gq * (e * psi1);
+    }
+    g = g + gh;
+    return energy;
 }
 
-// activation (src/ogc/potential.rs:8-22)
-template <class S>
-__device__ __forceinline__ S activation(const S& d, double r, double k) {
-    if (sval(d) >= r) return scst<S>(0.0);
-    if (sval(d) <= 0.0) return scst<S>(__longlong_as_double(0x7ff0000000000000ll));
-    double tau = 0.5 * r;
-    if (sval(d) >= tau) {
-        S gg = scst<S>(r) - d;
-        return scst<S>(0.5 * k) * gg * gg;
-    }
-    return scst<S>(0.5 * k * tau * tau) - scst<S>(k * tau * tau) * sln(d / scst<S>(tau));
-}
-
-// Contact distance of Contact::energy (src/ogc/potential.rs:39-65) on four
-// named points; `degenerate` is set for an EE pair with |n|^2 < 1e-30 (energy 0).
-template <class S>
-__device__ __forceinline__ S contact_distance(uint32_t kind, const V<S>& p0, const V<S>& p1, const V<S>& p2,
-                                              const V<S>& p3, bool& degenerate) {
-    degenerate = false;
-    if (kind == 0) {
-        V<S> v = vsub(p0, p1);
-        return ssqrt(vdot(v, v));
-    }
-    if (kind == 1) {
-        V<S> u = vsub(p2, p1);
-        V<S> w = vsub(p0, p1);
-        S q = vdot(w, u) / vdot(u, u);
-        V<S> dd = {w.x - q * u.x, w.y - q * u.y, w.z - q * u.z};
-        return ssqrt(vdot(dd, dd));
-    }
-    if (kind == 2) {
-        V<S> n = vcross(vsub(p2, p1), vsub(p3, p1));
-        S h = vdot(vsub(p0, p1), n) / ssqrt(vdot(n, n));
-        return sval(h) < 0.0 ? -h : h;
-    }
-    V<S> n = vcross(vsub(p1, p0), vsub(p3, p2));
-    if (sval(vdot(n, n)) < 1e-30) {
-        degenerate = true;
-        return scst<S>(0.0);
-    }
-    S h = vdot(vsub(p0, p2), n) / ssqrt(vdot(n, n));
-    return sval(h) < 0.0 ? -h : h;
-}
-
-// Contact::energy (src/ogc/potential.rs:39-65) on four named points.
-template <class S>
-__device__ __forceinline__ S contact_energy_t(uint32_t kind, double eps, const V<S>& p0, const V<S>& p1,
-                                              const V<S>& p2, const V<S>& p3, double r, double k) {
-    bool degenerate;
-    S d = contact_distance<S>(kind, p0, p1, p2, p3, degenerate);
-    if (degenerate) return scst<S>(0.0);
-    S e = activation(d, r, k);
-    if (kind == 3) {
-        V<S> n = vcross(vsub(p1, p0), vsub(p3, p2));
-        S q = vdot(n, n) / scst<S>(eps);
-        if (sval(q) < 1.0) e = e * q * (scst<S>(2.0) - q);
-    }
-    return e;
-}
-
-// ---- mixed Jet/constant arithmetic: only the moving vertex carries derivatives
-__device__ __forceinline__ J3 operator+(const J3& a, double b) {
-    J3 r = a;
-    r.v += b;
-    return r;
-}
-__device__ __forceinline__ J3 operator+(double a, const J3& b) { return b + a; }
-__device__ __forceinline__ J3 operator-(const J3& a, double b) {
-    J3 r = a;
-    r.v -= b;
-    return r;
-}
-__device__ __forceinline__ J3 operator-(double a, const J3& b) {
-    J3 r = -b;
-    r.v += a;
-    return r;
-}
-__device__ __forceinline__ J3 operator*(const J3& a, double b) {
-    return {a.v * b, a.g0 * b, a.g1 * b, a.g2 * b, a.h00 * b, a.h01 * b, a.h02 * b, a.h11 * b, a.h12 * b, a.h22 * b};
-}
-__device__ __forceinline__ J3 operator*(double a, const J3& b) { return b * a; }
-__device__ __forceinline__ J3 operator/(const J3& a, double b) { return a * (1.0 / b); }
-__device__ __forceinline__ J3 operator/(double a, const J3& b) {
-    return chain(b, 1.0 / b.v, -1.0 / (b.v * b.v), 2.0 / (b.v * b.v * b.v)) * a;
-}
-__device__ __forceinline__ J3 to_j3(const J3& a) { return a; }
-__device__ __forceinline__ J3 to_j3(double a) { return jc(a); }
-
-template <class A, class B>
-struct Pro {
-    using T = J3;
-};
-template <>
-struct Pro<double, double> {
-    using T = double;
-};
-template <class A, class B>
-__device__ __forceinline__ V<typename Pro<A, B>::T> msub(const V<A>& a, const V<B>& b) {
-    return {a.x - b.x, a.y - b.y, a.z - b.z};
-}
-template <class A, class B>
-__device__ __forceinline__ typename Pro<A, B>::T mdot(const V<A>& a, const V<B>& b) {
-    return a.x * b.x + a.y * b.y + a.z * b.z;
-}
-template <class A, class B>
-__device__ __forceinline__ V<typename Pro<A, B>::T> mcross(const V<A>& a, const V<B>& b) {
-    return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
-}
-
-// Contact::energy (src/ogc/potential.rs:39-65) with per-point types.
-template <class S0, class S1, class S2, class S3>
-__device__ __forceinline__ J3 contact_jet(uint32_t kind, double eps, const V<S0>& p0, const V<S1>& p1,
-                                          const V<S2>& p2, const V<S3>& p3, double r, double k) {
-    if (kind == 0) {
-        auto v = msub(p0, p1);
-        return to_j3(activation(ssqrt(mdot(v, v)), r, k));
-    }
-    if (kind == 1) {
-        auto u = msub(p2, p1);
-        auto w = msub(p0, p1);
-        auto q = mdot(w, u) / mdot(u, u);
-        auto dx = w.x - q * u.x;
-        auto dy = w.y - q * u.y;
-        auto dz = w.z - q * u.z;
-        return to_j3(activation(ssqrt(dx * dx + dy * dy + dz * dz), r, k));
-    }
-    if (kind == 2) {
-        auto n = mcross(msub(p2, p1), msub(p3, p1));
-        auto h = mdot(msub(p0, p1), n) / ssqrt(mdot(n, n));
-        auto d = sval(h) < 0.0 ? -h : h;
-        return to_j3(activation(d, r, k));
-    }
-    auto n = mcross(msub(p1, p0), msub(p3, p2));
-    auto nn = mdot(n, n);
-    if (sval(nn) < 1e-30) return jc(0.0);
-    auto h = mdot(msub(p0, p2), n) / ssqrt(nn);
-    auto d = sval(h) < 0.0 ? -h : h;
-    J3 e = to_j3(activation(d, r, k));
-    J3 q = to_j3(nn / eps);
-    if (q.v < 1.0) e = e * q * (2.0 - q);
-    return e;
-}
-
-__device__ __forceinline__ V<J3> var_point(d3 p) {
-    J3 a = jc(p.x), b = jc(p.y), c = jc(p.z);
-    a.g0 = 1.0;
-    b.g1 = 1.0;
-    c.g2 = 1.0;
-    return {a, b, c};
-}
-__device__ __forceinline__ V<double> cst_point(const SweepView& s, uint32_t id) {
-    d3 x = ld3(s.x, id);
-    return {x.x, x.y, x.z};
-}
-__device__ __forceinline__ V<double> dpoint(const SweepView& s, uint32_t id, uint32_t v, d3 p) {
-    d3 x = pos(s, id, v, p);
-    return {x.x, x.y, x.z};
-}
-
-template <bool D>
-__device__ __forceinline__ double contact_term(const SweepView& s, uint32_t c, uint32_t v, d3 p, d3& g, Sym& H) {
-    uint32_t kind = s.contacts.kind[c];
-    uint4 cv = s.contacts.verts[c];
-    double eps = s.contacts.eps[c];
-    if (D) {
-        // Inactive term (d >= r): the activation is the constant 0, so the term
-        // adds nothing to e, g or H; skip its derivative evaluation.
-        bool degenerate;
-        double d0 = contact_distance<double>(kind, dpoint(s, cv.x, v, p), dpoint(s, cv.y, v, p),
-                                             dpoint(s, cv.z, v, p), dpoint(s, cv.w, v, p), degenerate);
-        if (degenerate || d0 >= s.contact_r) return 0.0;
-        // the moving vertex's slot among the used ones (unused slots hold 0)
-        uint32_t cnt = kind == 0 ? 2u : (kind == 1 ? 3u : 4u);
-        int slot = cv.x == v ? 0 : (cv.y == v ? 1 : ((cnt > 2 && cv.z == v) ? 2 : 3));
-        double r = s.contact_r, k = s.contact_k;
-        J3 e;
-        if (slot == 0)
-            e = contact_jet(kind, eps, var_point(p), cst_point(s, cv.y), cst_point(s, cv.z), cst_point(s, cv.w), r, k);
-        else if (slot == 1)
-            e = contact_jet(kind, eps, cst_point(s, cv.x), var_point(p), cst_point(s, cv.z), cst_point(s, cv.w), r, k);
-        else if (slot == 2)
-            e = contact_jet(kind, eps, cst_point(s, cv.x), cst_point(s, cv.y), var_point(p), cst_point(s, cv.w), r, k);
-        else
-            e = contact_jet(kind, eps, cst_point(s, cv.x), cst_point(s, cv.y), cst_point(s, cv.z), var_point(p), r, k);
-        g = g + mk(e.g0, e.g1, e.g2);
-        H.a[0] += e.h00;
-        H.a[1] += e.h01;
-        H.a[2] += e.h02;
-        H.a[3] += e.h11;
-        H.a[4] += e.h12;
-        H.a[5] += e.h22;
-        return e.v;
-    }
-    return contact_energy_t<double>(kind, eps, dpoint(s, cv.x, v, p), dpoint(s, cv.y, v, p), dpoint(s, cv.z, v, p),
-                                    dpoint(s, cv.w, v, p), s.contact_r, s.contact_k);
+// energy of contact c alone
+__device__ __forceinline__ double contact_energy(const SweepView& s, uint32_t c) {
+    const uint4 v = s.contacts.verts[c];
+    d3 g;
+    Sym H;
+    return contact_rec<false>(s, contact_ref(s.contacts.kind[c], v, v.x), s.contacts.eps[c], ld3(s.x, v.x), g, H);
 }
 
 // grab 0.5 k |sum w_j x_j - target|^2 (src/vbd.rs:237-246)
@@ -497,79 +351,139 @@ __device__ __forceinline__ double grab_term(const SweepView& s, uint32_t v, d3 p
     return 0.5 * G.k * dot(d, d);
 }
 
+// A vertex's terms with its neighbours' positions staged in shared memory, one
+// column of kSlots positions per group of G lanes (an interior grid vertex has 12
+// neighbours; further ones are read from global memory). A position is read
+// once, by one lane, and all the terms of the derivative pass and of every
+// line-search trial take it from there.
+template <int G>
+struct Near {
+    static constexpr uint32_t kSlots = G >= 4 ? 24 : (G == 2 ? 16 : 8);
+    static constexpr uint32_t kDoubles = 3 * kSlots;  // per group
+    uint32_t v, nb0, n_nb, t0, nt, h0, ne, nw, ns, c0, c1;
+    double* at;  // x, y and z of the staged positions
+
+    // A lane's first record of each kind, loaded while the neighbours' ids and
+    // positions are on their way; the loops of local_part load the next round's
+    // records before they evaluate the present one.
+    struct First {
+        unsigned long long t;
+        double4 tb, tk;
+        ulonglong2 edge, wing;
+        uint4 c;
+        double eps;
+    };
+
+    __device__ __forceinline__ void head(const SweepView& s, uint32_t vertex) {
+        v = vertex;
+        const uint4 a = s.vt.head[2 * (size_t)v], b = s.vt.head[2 * (size_t)v + 1];
+        nb0 = a.x, n_nb = a.y, t0 = a.z, nt = a.w;
+        h0 = b.x, ne = b.y, nw = b.z, ns = b.w;
+        c0 = s.contacts.inc_off[v];
+        c1 = s.contacts.inc_off[v + 1];
+    }
+    // head i of the colour (k_color_heads)
+    __device__ __forceinline__ void head_of_color(const SweepView& s, uint32_t i) {
+        const uint4 a = s.heads[3 * (size_t)i], b = s.heads[3 * (size_t)i + 1], c = s.heads[3 * (size_t)i + 2];
+        v = a.x, nb0 = a.y, n_nb = a.z, t0 = a.w;
+        nt = b.x, h0 = b.y, ne = b.z, nw = b.w;
+        ns = c.x, c0 = c.y, c1 = c.z;
+    }
+    __device__ __forceinline__ void tri(const SweepView& s, uint32_t i, First& f) const {
+        if (i < nt) {
+            f.t = s.vt.tri[t0 + i];
+            f.tb = s.vt.tri_b[t0 + i];
+            f.tk = s.vt.tri_k[t0 + i];
+        }
+    }
+    __device__ __forceinline__ void contact(const SweepView& s, uint32_t k, First& f) const {
+        if (k < c1) {
+            f.c = s.contacts.ref[k];
+            f.eps = s.contacts.ref_eps[k];
+        }
+    }
+    __device__ __forceinline__ First first(const SweepView& s, uint32_t lane) const {
+        First f{};
+        tri(s, lane, f);
+        if (lane < ne) f.edge = s.vt.hinge[h0 + lane];
+        if (lane < nw) f.wing = s.vt.hinge[h0 + ne + lane];
+        contact(s, c0 + lane, f);
+        return f;
+    }
+    // The first records, and the neighbours' positions into shared memory; the
+    // whole group calls it.
+    __device__ __forceinline__ First load(const SweepView& s, uint32_t lane, unsigned mask, double* smem) {
+        at = smem;
+        constexpr int J = (kSlots + G - 1) / G;
+        const uint32_t m = min(n_nb, kSlots);
+        uint32_t id[J];
+        d3 q[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) id[j] = lane + j * G < m ? s.vt.nb[nb0 + lane + j * G] : 0u;
+        const First f = first(s, lane);
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            if (lane + j * G < m) q[j] = ld3(s.x, id[j]);
+        __syncwarp(mask);  // the column's last reads are done
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const uint32_t k = lane + j * G;
+            if (k < m) {
+                at[k] = q[j].x;
+                at[kSlots + k] = q[j].y;
+                at[2 * kSlots + k] = q[j].z;
+            }
+        }
+        __syncwarp(mask);
+        return f;
+    }
+    __device__ __forceinline__ d3 pos(const SweepView& s, uint32_t i) const {
+        if (i < kSlots) return mk(at[i], at[kSlots + i], at[2 * kSlots + i]);
+        return ld3(s.x, s.vt.nb[nb0 + i]);
+    }
+};
+
 // Partial sum of the incident terms dealt to `lane` of a group of G
-// (VbdSolver::local, src/vbd.rs:196-248).
+// (VbdSolver::local, src/vbd.rs:196-248), with the vertex at p; f holds the
+// lane's first records.
 template <bool D, int G, bool HS = D>
-__device__ __forceinline__ double local_part(const SweepView& s, uint32_t v, d3 p, uint32_t lane, d3& g, Sym& H) {
+__device__ __forceinline__ double local_part(const SweepView& s, const Near<G>& T, typename Near<G>::First f, d3 p,
+                                             uint32_t lane, d3& g, Sym& H) {
+    constexpr uint32_t kId = (1u << 21) - 1u;
     double e = 0.0;
-    // entries are grouped by type: one lane-strided loop per type, no per-entry dispatch
-    uint32_t b0 = s.inc_off[v], b1 = s.inc_off[v + 1];
-    uint2 mid = s.inc_mid[v];
-    // each loop loads the next term's record before it evaluates the current one
-    {
-        uint32_t k = b0 + lane;
-        uint32_t ent = k < mid.x ? s.inc[k] : 0u;
-        int4 tv = make_int4(0, 0, 0, 0);
-        double4 cf = make_double4(0, 0, 0, 0);
-        double A = 0.0;
-        if (k < mid.x) {
-            uint32_t t = ent & 0x0fffffffu;
-            tv = s.tri_v[t];
-            cf = s.tri_coef[t];
-            A = s.tri_area[t];
-        }
-        for (; k < mid.x; k += G) {
-            uint32_t kn = k + G;
-            uint32_t en = 0u;
-            int4 tvn = tv;
-            double4 cfn = cf;
-            double An = A;
-            if (kn < mid.x) {
-                en = s.inc[kn];
-                uint32_t t = en & 0x0fffffffu;
-                tvn = s.tri_v[t];
-                cfn = s.tri_coef[t];
-                An = s.tri_area[t];
-            }
-            e += membrane_rec<D, HS>(s, tv, cf, A, (ent >> 28) & 3u, p, g, H);
-            ent = en;
-            tv = tvn;
-            cf = cfn;
-            A = An;
-        }
+    for (uint32_t i = lane; i < T.nt; i += G) {
+        const unsigned long long t = f.t;
+        const double4 b = f.tb, k = f.tk;
+        T.tri(s, i + G, f);
+        e += membrane<D, HS>(s, b, k, (uint32_t)(t >> 42), T.pos(s, (uint32_t)t & kId) - p,
+                             T.pos(s, (uint32_t)(t >> 21) & kId) - p, g, H);
     }
-    {
-        uint32_t k = mid.x + lane;
-        uint32_t ent = k < mid.y ? s.inc[k] : 0u;
-        uint4 hv = make_uint4(0, 0, 0, 0);
-        double K = 0.0;
-        if (k < mid.y) {
-            uint32_t h = ent & 0x0fffffffu;
-            hv = s.hinge_v[h];
-            K = s.hinge_k[h];
-        }
-        for (; k < mid.y; k += G) {
-            uint32_t kn = k + G;
-            uint32_t en = 0u;
-            uint4 hvn = hv;
-            double Kn = K;
-            if (kn < mid.y) {
-                en = s.inc[kn];
-                uint32_t h = en & 0x0fffffffu;
-                hvn = s.hinge_v[h];
-                Kn = s.hinge_k[h];
-            }
-            e += bending_rec<D, HS>(s, hv, K, (ent >> 28) & 3u, p, g, H);
-            ent = en;
-            hv = hvn;
-            K = Kn;
-        }
+    // edge ends, then wings: the lanes of a round take the same form
+    for (uint32_t i = lane; i < T.ne; i += G) {
+        const ulonglong2 h = f.edge;
+        if (i + G < T.ne) f.edge = s.vt.hinge[T.h0 + i + G];
+        e += bending_edge<D, HS>(__longlong_as_double((long long)h.y), T.pos(s, (uint32_t)h.x & kId),
+                                 T.pos(s, (uint32_t)(h.x >> 21) & kId), T.pos(s, (uint32_t)(h.x >> 42)), p, g, H);
     }
-    for (uint32_t k = mid.y + lane; k < b1; k += G) e += stitch_term<D>(s, s.inc[k] & 0x0fffffffu, v, p, g, H);
-    uint32_t c1 = s.contacts.inc_off[v + 1];
-    for (uint32_t k = s.contacts.inc_off[v] + lane; k < c1; k += G) e += contact_term<D>(s, s.contacts.inc[k], v, p, g, H);
-    if (lane == 0 && s.grab.active && (s.grab.v[0] == v || s.grab.v[1] == v || s.grab.v[2] == v))
-        e += grab_term<D>(s, v, p, g, H);
+    for (uint32_t i = lane; i < T.nw; i += G) {
+        const ulonglong2 h = f.wing;
+        if (i + G < T.nw) f.wing = s.vt.hinge[T.h0 + T.ne + i + G];
+        e += bending_wing<D, HS>(__longlong_as_double((long long)h.y), T.pos(s, (uint32_t)h.x & kId),
+                                 T.pos(s, (uint32_t)(h.x >> 21) & kId), T.pos(s, (uint32_t)(h.x >> 42)), p, g, H);
+    }
+    if (T.ns) {
+        const uint32_t b1 = s.inc_off[T.v + 1];
+        for (uint32_t k = b1 - T.ns + lane; k < b1; k += G)
+            e += stitch_term<D>(s, s.inc[k] & 0x0fffffffu, T.v, p, g, H);
+    }
+    for (uint32_t k = T.c0 + lane; k < T.c1; k += G) {
+        const uint4 c = f.c;
+        const double eps = f.eps;
+        T.contact(s, k + G, f);
+        e += contact_rec<D, HS>(s, c, eps, p, g, H);
+    }
+    if (lane == 0 && s.grab.active && (s.grab.v[0] == T.v || s.grab.v[1] == T.v || s.grab.v[2] == T.v))
+        e += grab_term<D>(s, T.v, p, g, H);
     return e;
 }
 

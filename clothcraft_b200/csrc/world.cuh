@@ -99,6 +99,29 @@ struct DetectStats {  // read back after each detection
     unsigned int rebuild;
 };
 
+// The part a vertex plays in a contact, with the other points' order:
+//   POINT (PP): {q}                        distance |p - q|
+//   FROM_LINE (PE, the point): {a, b}      distance of p from the line a b
+//   ON_LINE (PE, an end): {other end, point}
+//   FROM_PLANE (PF, the point): {a, b, c}  distance of p from the plane a b c
+//   ON_PLANE (PF, a corner): {j, k, point} distance of the point from the plane p j k
+//   EDGES (EE): {other end of p's edge, c, d}
+enum ContactRole : uint32_t { POINT = 0, FROM_LINE = 1, ON_LINE = 2, FROM_PLANE = 3, ON_PLANE = 4, EDGES = 5 };
+// contact (kind, vertices) as seen from its vertex v: points in x, y, z, role in w
+__device__ __forceinline__ uint4 contact_ref(uint32_t kind, uint4 c, uint32_t v) {
+    if (kind == 0) return make_uint4(c.x == v ? c.y : c.x, 0u, 0u, POINT);
+    if (kind == 1) {
+        if (c.x == v) return make_uint4(c.y, c.z, 0u, FROM_LINE);
+        return make_uint4(c.y == v ? c.z : c.y, c.x, 0u, ON_LINE);
+    }
+    if (kind == 2) {
+        if (c.x == v) return make_uint4(c.y, c.z, c.w, FROM_PLANE);
+        return make_uint4(c.y == v ? c.z : c.y, c.w == v ? c.z : c.w, c.x, ON_PLANE);
+    }
+    if (c.x == v || c.y == v) return make_uint4(c.x == v ? c.y : c.x, c.z, c.w, EDGES);
+    return make_uint4(c.z == v ? c.w : c.z, c.x, c.y, EDGES);
+}
+
 struct ContactsView {  // canonical contact set for the sweep and colouring
     uint32_t n;
     const uint32_t* kind;   // [n]
@@ -106,6 +129,8 @@ struct ContactsView {  // canonical contact set for the sweep and colouring
     const double* eps;      // [n]
     const uint32_t* inc_off;  // [moving+1]
     const uint32_t* inc;      // contact ids
+    const uint4* ref;         // [entries of inc] the contact as its row's vertex sees it: points (x, y, z), role (w)
+    const double* ref_eps;    // [entries of inc] its mollifier epsilon
     const double4* centers;   // [moving]
     const double* radii;      // [moving]
 };
@@ -207,7 +232,9 @@ class World {
     DBuf<unsigned long long> dist_bits_;
     DBuf<double> radii_;
     DBuf<double4> centers_;
-    DBuf<uint32_t> inc_count_, inc_off_, inc_, inc_cursor_;
+    DBuf<uint32_t> inc_count_, inc_off_, inc_, inc_raw_, inc_cursor_;
+    DBuf<uint4> inc_ref_;
+    DBuf<double> inc_eps_;
     RadixSorter sorter_;
     DBuf<uint32_t> scan_tmp_;
     DBuf<DetectStats> stats_d_;
