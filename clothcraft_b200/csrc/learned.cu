@@ -19,6 +19,7 @@
 // guess + u * c, clipped to the vertex's OGC ball.
 #include <cuda_fp16.h>
 
+#include <atomic>
 #include <cmath>
 #include <vector>
 
@@ -237,162 +238,235 @@ __global__ void __launch_bounds__(kFwdBlock) k_mlp_forward_f32(const float* __re
 }
 
 // ------------------------------------------------------------- training
-// One CTA of 128 threads processes tiles of 64 samples: forward (two threads
-// per sample, 32 units each), loss gradient, back-propagation, and the
-// weight gradients of the tile (sum over its samples) added to the CTA's own
-// row of `partial`; k_mlp_reduce then sums the rows in a fixed order.
+// One CTA of 256 threads per SM processes tiles of up to 64 samples: forward,
+// loss gradient and back-propagation with every operand in shared memory, the
+// weight gradients summed over the CTA's tiles in registers and written once
+// into the CTA's row of `partial`; k_mlp_reduce sums the rows in a fixed order.
+//
+// All three products are FP32 FMA (no tensor-core format keeps FP32 operands),
+// so the bound is 6 x 9,920 operations a sample: 16,384 samples are 13 us at
+// ~75 TFLOP/s. A thread owns a 4 x 4 block of the result and reads two float4
+// per 16 FMAs: weights transposed for the forward pass ([in][out]) and as they
+// are for the backward one, activations unit-major (a row of kPitch samples), so
+// that both sides of every product are contiguous float4. One thread per sample
+// and unit range, weights from global memory and one weight gradient per thread
+// at two shared-memory reads per FMA, took 290 us for the 16,384.
 constexpr int kTile = 64;
-constexpr int kPitch = kTile + 1;  // row pitch: unit-major rows, one column per sample
-constexpr int kTrainBlock = 128;
-constexpr int kTrainFloats = kMlpIn * kPitch + 6 * kMlpHidden * kPitch + 2 * kMlpHidden * kPitch + kMlpOut * kPitch;
+constexpr int kPitch = kTile + 4;  // float4 rows; rows r and r + 1 lie 4 banks apart
+constexpr int kTrainBlock = 256;
+constexpr int kWPitch = kMlpHidden + 4;
+// shared memory (floats): weights, then activations
+constexpr int kSmW2 = 0;
+constexpr int kSmW3 = kSmW2 + kMlpHidden * kMlpHidden;
+constexpr int kSmW4 = kSmW3 + kMlpHidden * kMlpHidden;
+constexpr int kSmT1 = kSmW4 + kMlpOut * kMlpHidden;
+constexpr int kSmT2 = kSmT1 + kMlpIn * kWPitch;
+constexpr int kSmT3 = kSmT2 + kMlpHidden * kWPitch;
+constexpr int kSmB = kSmT3 + kMlpHidden * kWPitch;  // b1 b2 b3 b4 (+ 1)
+constexpr int kSmX = kSmB + 3 * kMlpHidden + 4;
+constexpr int kSmA1 = kSmX + kMlpIn * kPitch;  // activations A and GELU derivatives G, later the deltas in G's place
+constexpr int kSmLayer = kMlpHidden * kPitch;
+constexpr int kSmG1 = kSmA1 + kSmLayer, kSmA2 = kSmG1 + kSmLayer, kSmG2 = kSmA2 + kSmLayer;
+constexpr int kSmA3 = kSmG2 + kSmLayer, kSmG3 = kSmA3 + kSmLayer, kSmD4 = kSmG3 + kSmLayer;
+constexpr int kTrainFloats = kSmD4 + kMlpOut * kPitch;
+static_assert(kSmX % 4 == 0 && kSmT1 % 4 == 0 && kTrainFloats * 4 <= 227 * 1024, "float4 rows, one block per SM");
 
-__device__ __forceinline__ void add_partial(float* row, int p, float v) { row[p] += v; }
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
+    *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+// acc[i][j] += w[i] * a[j]
+__device__ __forceinline__ void outer4(float (&acc)[4][4], float4 w, float4 a) {
+    const float wv[4] = {w.x, w.y, w.z, w.w}, av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(wv[i], av[j], acc[i][j]);
+}
 
-// dW[o][i] += sum_s D[o][s] * A[i][s]; db[o] += sum_s D[o][s]
-__device__ __forceinline__ void weight_grads(const float* D, const float* A, int outs, int ins, int valid, float* row,
-                                             int offW, int offB) {
-    int entries = outs * ins + outs;
-    for (int e = threadIdx.x; e < entries; e += kTrainBlock) {
-        float acc = 0.0f;
-        if (e < outs * ins) {
-            int o = e / ins, i = e - o * ins;
-            const float* d = D + o * kPitch;
-            const float* a = A + i * kPitch;
-            for (int s = 0; s < valid; ++s) acc = fmaf(d[s], a[s], acc);
-            add_partial(row, offW + e, acc);
-        } else {
-            int o = e - outs * ins;
-            const float* d = D + o * kPitch;
-            for (int s = 0; s < valid; ++s) acc += d[s];
-            add_partial(row, offB + o, acc);
+// hidden layer, units u0..u0+3 of samples s0..s0+3: A = gelu(W in + b), G = gelu'
+template <int IN>
+__device__ __forceinline__ void train_forward(const float* wt, const float* b, const float* in, int u0, int s0, float* A,
+                                              float* G) {
+    float z[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) z[i][j] = b[u0 + i];
+#pragma unroll 8
+    for (int k = 0; k < IN; ++k) outer4(z, ld4(wt + k * kWPitch + u0), ld4(in + k * kPitch + s0));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float a[4], d[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) gelu_fg(z[i][j], a[j], d[j]);
+        st4(A + (u0 + i) * kPitch + s0, a[0], a[1], a[2], a[3]);
+        st4(G + (u0 + i) * kPitch + s0, d[0], d[1], d[2], d[3]);
+    }
+}
+
+// deltas of a hidden layer in the place of its GELU derivatives: G[i][s] *= sum_o W[o][i] D[o][s]
+template <int OUTS>
+__device__ __forceinline__ void train_backward(const float* w, const float* D, int u0, int s0, float* G) {
+    float acc[4][4] = {};
+#pragma unroll 8
+    for (int o = 0; o < OUTS; ++o) outer4(acc, ld4(w + o * kMlpHidden + u0), ld4(D + o * kPitch + s0));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float* g = G + (u0 + i) * kPitch + s0;
+        const float4 d = ld4(g);
+        st4(g, d.x * acc[i][0], d.y * acc[i][1], d.z * acc[i][2], d.w * acc[i][3]);
+    }
+}
+
+// acc[a][b] += sum_s D[4 og + a][s] A[ig + 16 b][s]: the weight gradients of outputs 4 og + a, inputs ig + 16 b
+template <int NB>
+__device__ __forceinline__ void train_weights(const float* D, const float* A, int og, int ig, int tile, int nb,
+                                              float (&acc)[4][NB]) {
+    for (int s = 0; s < tile; s += 4) {
+        float4 d[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) d[a] = ld4(D + (4 * og + a) * kPitch + s);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            if (b >= nb) break;
+            const float4 x = ld4(A + (ig + 16 * b) * kPitch + s);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                acc[a][b] = fmaf(d[a].x, x.x, acc[a][b]);
+                acc[a][b] = fmaf(d[a].y, x.y, acc[a][b]);
+                acc[a][b] = fmaf(d[a].z, x.z, acc[a][b]);
+                acc[a][b] = fmaf(d[a].w, x.w, acc[a][b]);
+            }
         }
     }
 }
 
-// forward of one hidden layer for sample s, units [u0, u0+32)
-template <int IN>
-__device__ __forceinline__ void fwd_half(const float* __restrict__ P, int offW, int offB, const float* in_rows, int s,
-                                         int u0, float* A, float* G) {
-    float x[IN];
-#pragma unroll
-    for (int j = 0; j < IN; ++j) x[j] = in_rows[j * kPitch + s];
-#pragma unroll 1
-    for (int i = u0; i < u0 + 32; ++i) {
-        float z = P[offB + i];
-        const float* wr = P + offW + i * IN;
-#pragma unroll
-        for (int j = 0; j < IN; ++j) z = fmaf(wr[j], x[j], z);
-        float a, da;
-        gelu_fg(z, a, da);
-        A[i * kPitch + s] = a;
-        G[i * kPitch + s] = da;
-    }
-}
-
-// delta of a hidden layer: Dout[i][s] = G[i][s] * sum_o W[o][i] Din[o][s], i in [u0, u0+32)
-template <int OUTS>
-__device__ __forceinline__ void bwd_half(const float* __restrict__ P, int offW, const float* Din, const float* G, int s,
-                                         int u0, float* Dout) {
-    float d[OUTS];
-#pragma unroll
-    for (int o = 0; o < OUTS; ++o) d[o] = Din[o * kPitch + s];
-#pragma unroll 1
-    for (int i = u0; i < u0 + 32; ++i) {
-        float acc = 0.0f;
-#pragma unroll
-        for (int o = 0; o < OUTS; ++o) acc = fmaf(P[offW + o * kMlpHidden + i], d[o], acc);
-        Dout[i * kPitch + s] = G[i * kPitch + s] * acc;
-    }
-}
-
+// `tile`: samples per tile, a multiple of 4 up to kTile
 __global__ void __launch_bounds__(kTrainBlock) k_mlp_train_tile(const float* __restrict__ P, const float* __restrict__ F,
                                                                   const float* __restrict__ T,
                                                                   const uint32_t* __restrict__ index, uint64_t n,
-                                                                  float inv_n, float* partial) {
-    extern __shared__ float sm[];
-    float* X = sm;                                // [24][pitch]
-    float* A1 = X + kMlpIn * kPitch;              // [64][pitch] activations
-    float* G1 = A1 + kMlpHidden * kPitch;         // [64][pitch] GELU derivatives
-    float* A2 = G1 + kMlpHidden * kPitch;
-    float* G2 = A2 + kMlpHidden * kPitch;
-    float* A3 = G2 + kMlpHidden * kPitch;
-    float* G3 = A3 + kMlpHidden * kPitch;
-    float* Da = G3 + kMlpHidden * kPitch;         // [64][pitch] deltas (ping)
-    float* Db = Da + kMlpHidden * kPitch;         // (pong)
-    float* D4 = Db + kMlpHidden * kPitch;         // [3][pitch]
-    float* row = partial + (size_t)blockIdx.x * (kMlpParams + 1);
-    const int s = threadIdx.x & (kTile - 1);
-    const int half = threadIdx.x >> 6;  // 0 or 1
-    const uint64_t tiles = (n + kTile - 1) / kTile;
-    float loss = 0.0f;
-    for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        uint64_t base = tile * kTile;
-        int valid = (int)(n - base < (uint64_t)kTile ? n - base : (uint64_t)kTile);
-        // inputs (zero columns past the end)
-        for (int e = threadIdx.x; e < kMlpIn * kTile; e += kTrainBlock) {
-            int ss = e / kMlpIn, j = e - ss * kMlpIn;
+                                                                  int tile, float inv_n, float* partial) {
+    extern __shared__ __align__(16) float sm[];
+    const int t = threadIdx.x;
+    for (int e = t; e < kMlpHidden * kMlpHidden; e += kTrainBlock) {
+        const int o = e / kMlpHidden, k = e % kMlpHidden;
+        const float w2 = P[kOffW2 + e], w3 = P[kOffW3 + e];
+        sm[kSmW2 + e] = w2;
+        sm[kSmW3 + e] = w3;
+        sm[kSmT2 + k * kWPitch + o] = w2;
+        sm[kSmT3 + k * kWPitch + o] = w3;
+    }
+    for (int e = t; e < kMlpHidden * kMlpIn; e += kTrainBlock)
+        sm[kSmT1 + (e % kMlpIn) * kWPitch + e / kMlpIn] = P[kOffW1 + e];
+    if (t < kMlpOut * kMlpHidden) sm[kSmW4 + t] = P[kOffW4 + t];
+    if (t < kMlpHidden) {
+        sm[kSmB + t] = P[kOffB1 + t];
+        sm[kSmB + kMlpHidden + t] = P[kOffB2 + t];
+        sm[kSmB + 2 * kMlpHidden + t] = P[kOffB3 + t];
+    }
+    if (t < kMlpOut) sm[kSmB + 3 * kMlpHidden + t] = P[kOffB4 + t];
+    const int u0 = 4 * (t >> 4), s0 = 4 * (t & 15), og = t >> 4, ig = t & 15;
+    // gradients of this thread: its 4 x 4 blocks of W2 and W3, 4 x 2 of W1, one entry of W4 and one bias
+    float g1[4][2] = {}, g2[4][4] = {}, g3[4][4] = {}, g4 = 0.0f, gb = 0.0f, loss = 0.0f;
+    const int nb1 = ig < kMlpIn - 16 ? 2 : 1;
+    const float* bias_rows = t < 64 ? sm + kSmG1 + t * kPitch
+                                    : (t < 128 ? sm + kSmG2 + (t - 64) * kPitch
+                                               : (t < 192 ? sm + kSmG3 + (t - 128) * kPitch
+                                                          : sm + kSmD4 + (t < 195 ? t - 192 : 0) * kPitch));
+    const uint64_t tiles = (n + tile - 1) / tile;
+    for (uint64_t k = blockIdx.x; k < tiles; k += gridDim.x) {
+        const uint64_t base = k * tile;
+        const int valid = (int)(n - base < (uint64_t)tile ? n - base : (uint64_t)tile);
+        __syncthreads();  // the weights are in place; the last tile is done with
+        for (int e = t; e < kMlpIn * tile; e += kTrainBlock) {  // zero columns past the end
+            const int ss = e / kMlpIn, j = e - ss * kMlpIn;
             float v = 0.0f;
-            if (ss < valid) {
-                uint64_t id = index ? index[base + ss] : base + ss;
-                v = F[id * kMlpIn + j];
-            }
-            X[j * kPitch + ss] = v;
+            if (ss < valid) v = F[(index ? index[base + ss] : base + ss) * kMlpIn + j];
+            sm[kSmX + j * kPitch + ss] = v;
         }
         __syncthreads();
-        fwd_half<kMlpIn>(P, kOffW1, kOffB1, X, s, half * 32, A1, G1);
+        if (s0 < tile) train_forward<kMlpIn>(sm + kSmT1, sm + kSmB, sm + kSmX, u0, s0, sm + kSmA1, sm + kSmG1);
         __syncthreads();
-        fwd_half<kMlpHidden>(P, kOffW2, kOffB2, A1, s, half * 32, A2, G2);
+        if (s0 < tile)
+            train_forward<kMlpHidden>(sm + kSmT2, sm + kSmB + kMlpHidden, sm + kSmA1, u0, s0, sm + kSmA2, sm + kSmG2);
         __syncthreads();
-        fwd_half<kMlpHidden>(P, kOffW3, kOffB3, A2, s, half * 32, A3, G3);
+        if (s0 < tile)
+            train_forward<kMlpHidden>(sm + kSmT3, sm + kSmB + 2 * kMlpHidden, sm + kSmA2, u0, s0, sm + kSmA3,
+                                      sm + kSmG3);
         __syncthreads();
         // output layer and dL/dout = 2 (out - t) / n (zero past the end)
-        if (half == 0) {
-            float h[kMlpHidden];
-#pragma unroll
-            for (int j = 0; j < kMlpHidden; ++j) h[j] = A3[j * kPitch + s];
-            uint64_t id = s < valid ? (index ? index[base + s] : base + s) : 0;
-#pragma unroll
-            for (int k = 0; k < kMlpOut; ++k) {
-                float o = P[kOffB4 + k];
-#pragma unroll
-                for (int j = 0; j < kMlpHidden; ++j) o = fmaf(P[kOffW4 + k * kMlpHidden + j], h[j], o);
-                float d = 0.0f;
-                if (s < valid) {
-                    float r = o - T[id * kMlpOut + k];
-                    loss += r * r;
-                    d = 2.0f * r * inv_n;
-                }
-                D4[k * kPitch + s] = d;
+        if (t < kMlpOut * kTile && (t & (kTile - 1)) < tile) {
+            const int o = t / kTile, s = t & (kTile - 1);
+            float v = sm[kSmB + 3 * kMlpHidden + o];
+#pragma unroll 8
+            for (int j = 0; j < kMlpHidden; ++j) v = fmaf(sm[kSmW4 + o * kMlpHidden + j], sm[kSmA3 + j * kPitch + s], v);
+            float d = 0.0f;
+            if (s < valid) {
+                const uint64_t id = index ? index[base + s] : base + s;
+                const float r = v - T[id * kMlpOut + o];
+                loss += r * r;
+                d = 2.0f * r * inv_n;
             }
+            sm[kSmD4 + o * kPitch + s] = d;
         }
         __syncthreads();
-        weight_grads(D4, A3, kMlpOut, kMlpHidden, valid, row, kOffW4, kOffB4);
-        bwd_half<kMlpOut>(P, kOffW4, D4, G3, s, half * 32, Da);
+        if (s0 < tile) train_backward<kMlpOut>(sm + kSmW4, sm + kSmD4, u0, s0, sm + kSmG3);
+        if (t < kMlpOut * kMlpHidden) {
+            const float *d = sm + kSmD4 + t / kMlpHidden * kPitch, *a = sm + kSmA3 + t % kMlpHidden * kPitch;
+            for (int s = 0; s < tile; ++s) g4 = fmaf(d[s], a[s], g4);
+        }
         __syncthreads();
-        weight_grads(Da, A2, kMlpHidden, kMlpHidden, valid, row, kOffW3, kOffB3);
-        bwd_half<kMlpHidden>(P, kOffW3, Da, G2, s, half * 32, Db);
+        train_weights<4>(sm + kSmG3, sm + kSmA2, og, ig, tile, 4, g3);
+        if (s0 < tile) train_backward<kMlpHidden>(sm + kSmW3, sm + kSmG3, u0, s0, sm + kSmG2);
         __syncthreads();
-        weight_grads(Db, A1, kMlpHidden, kMlpHidden, valid, row, kOffW2, kOffB2);
-        bwd_half<kMlpHidden>(P, kOffW2, Db, G1, s, half * 32, Da);
+        train_weights<4>(sm + kSmG2, sm + kSmA1, og, ig, tile, 4, g2);
+        if (s0 < tile) train_backward<kMlpHidden>(sm + kSmW2, sm + kSmG2, u0, s0, sm + kSmG1);
         __syncthreads();
-        weight_grads(Da, X, kMlpHidden, kMlpIn, valid, row, kOffW1, kOffB1);
-        __syncthreads();
+        train_weights<2>(sm + kSmG1, sm + kSmX, og, ig, tile, nb1, g1);
+        for (int s = 0; s < tile; ++s) gb += bias_rows[s];
     }
+    float* row = partial + (size_t)blockIdx.x * (kMlpParams + 1);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            row[kOffW2 + (4 * og + a) * kMlpHidden + ig + 16 * b] = g2[a][b];
+            row[kOffW3 + (4 * og + a) * kMlpHidden + ig + 16 * b] = g3[a][b];
+        }
+        for (int b = 0; b < nb1; ++b) row[kOffW1 + (4 * og + a) * kMlpIn + ig + 16 * b] = g1[a][b];
+    }
+    if (t < kMlpOut * kMlpHidden) row[kOffW4 + t] = g4;
+    if (t < 64) row[kOffB1 + t] = gb;
+    else if (t < 128) row[kOffB2 + t - 64] = gb;
+    else if (t < 192) row[kOffB3 + t - 128] = gb;
+    else if (t < 195) row[kOffB4 + t - 192] = gb;
     // loss: fixed-order block sum into the last slot of the row
     __shared__ float red[kTrainBlock];
-    red[threadIdx.x] = loss;
+    red[t] = loss;
     __syncthreads();
     for (int o = kTrainBlock / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+        if (t < o) red[t] += red[t + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) row[kMlpParams] = red[0] * inv_n;
+    if (t == 0) row[kMlpParams] = red[0] * inv_n;
 }
 
-__global__ void k_mlp_reduce(const float* partial, int rows, float* grads, float* loss) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p <= kMlpParams; p += gridDim.x * blockDim.x) {
-        float a = 0.0f;
-        for (int r = 0; r < rows; ++r) a += partial[(size_t)r * (kMlpParams + 1) + p];
+// Column sums of the rows: 64 columns a block, four threads a column (rows r, r + 4, ...)
+constexpr int kReduceCols = 64, kReduceParts = 4;
+__global__ void __launch_bounds__(kReduceCols* kReduceParts) k_mlp_reduce(const float* partial, int rows, float* grads,
+                                                                          float* loss) {
+    __shared__ float part[kReduceParts][kReduceCols];
+    const int c = threadIdx.x % kReduceCols, q = threadIdx.x / kReduceCols;
+    const int p = blockIdx.x * kReduceCols + c;
+    float a = 0.0f;
+    if (p <= kMlpParams)
+#pragma unroll 4
+        for (int r = q; r < rows; r += kReduceParts) a += partial[(size_t)r * (kMlpParams + 1) + p];
+    part[q][c] = a;
+    __syncthreads();
+    if (q == 0 && p <= kMlpParams) {
+        a = (part[0][c] + part[1][c]) + (part[2][c] + part[3][c]);
         if (p < kMlpParams) grads[p] = a;
         else *loss = a;
     }
@@ -476,15 +550,20 @@ void Mlp::forward(const float* features, uint64_t n, float* out, int precision, 
 void Mlp::gradients(const float* features, const float* targets, const uint32_t* index, uint64_t n, float* grads,
                     float* loss, cudaStream_t st) {
     if (n == 0) throw Failure{CC_ERR_INVALID_ARGUMENT, "MLP gradients need at least one sample"};
-    size_t smem = (size_t)kTrainFloats * sizeof(float);
-    allow_dynamic_smem(k_mlp_train_tile, smem);
-    uint64_t tiles = (n + kTile - 1) / kTile;
+    constexpr size_t smem = (size_t)kTrainFloats * sizeof(float);
+    static std::atomic<uint64_t> raised{0};  // devices on which the limit is raised
+    allow_dynamic_smem_once(k_mlp_train_tile, smem, raised);
+    // the smallest tile (a multiple of 4) with which every SM takes as many tiles
+    // as 64-sample tiles would: 16,384 samples are 2 x 148 tiles of 56
+    const uint64_t rounds = (n + 148ull * kTile - 1) / (148ull * kTile);
+    const int tile = (int)(((n + 148ull * rounds - 1) / (148ull * rounds) + 3) & ~3ull);
+    const uint64_t tiles = (n + tile - 1) / tile;
     int rows = (int)std::min<uint64_t>(tiles, 148ull);
     partial_.reserve((size_t)rows * (kMlpParams + 1));
-    CC_CUDA(cudaMemsetAsync(partial_.ptr, 0, (size_t)rows * (kMlpParams + 1) * sizeof(float), st));
-    k_mlp_train_tile<<<rows, kTrainBlock, smem, st>>>(p_.ptr, features, targets, index, n, 1.0f / (float)n,
+    k_mlp_train_tile<<<rows, kTrainBlock, smem, st>>>(p_.ptr, features, targets, index, n, tile, 1.0f / (float)n,
                                                       partial_.ptr);
-    k_mlp_reduce<<<(kMlpParams + 256) / 256, 256, 0, st>>>(partial_.ptr, rows, grads, loss);
+    k_mlp_reduce<<<(kMlpParams + kReduceCols) / kReduceCols, kReduceCols * kReduceParts, 0, st>>>(partial_.ptr, rows,
+                                                                                                  grads, loss);
     CC_CUDA(cudaGetLastError());
 }
 
