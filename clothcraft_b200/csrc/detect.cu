@@ -1232,8 +1232,8 @@ WorldView World::view() const {
 }
 
 ContactsView World::contacts() const {
-    return {(uint32_t)stats_h_.ptr->n_contacts, c_kind_.ptr, c_verts_.ptr, c_eps_.ptr, inc_off_.ptr, inc_.ptr,
-            inc_ref_.ptr, inc_eps_.ptr, centers_.ptr, radii_.ptr};
+    return {(uint32_t)stats_h_.ptr->n_contacts, c_kind_.ptr, c_verts_.ptr, c_eps_.ptr, inc_off_.ptr, inc_,
+            inc_ref_, inc_eps_, centers_.ptr, radii_.ptr};
 }
 
 void World::refit(bool check_fixed) {
@@ -1461,17 +1461,21 @@ void World::detect(double query_radius, double radius, double relaxation, double
     }
     launches_ += exclusive_sum(inc_count_.ptr, inc_off_.ptr, moving_ + 1, scan_tmp_, stream_);
     size_t n_inc_bound = 4 * n_raw;  // at most 4 moving vertices per contact
-    inc_.reserve(std::max<size_t>(n_inc_bound, 1));
-    inc_raw_.reserve(std::max<size_t>(n_inc_bound, 1));
-    inc_ref_.reserve(std::max<size_t>(n_inc_bound, 1));
-    inc_eps_.reserve(std::max<size_t>(n_inc_bound, 1));
+    inc_buf_.reserve(2 * std::max<size_t>(n_inc_bound, 1));  // 16 + 8 + 4 + 4 bytes an entry
+    {
+        const size_t cap = inc_buf_.cap / 2;
+        inc_ref_ = inc_buf_.ptr;
+        inc_eps_ = reinterpret_cast<double*>(inc_ref_ + cap);
+        inc_ = reinterpret_cast<uint32_t*>(inc_eps_ + cap);
+        inc_raw_ = inc_ + cap;
+    }
     if (n_raw > 0) {
         k_incidence_scatter<<<grid_for(n_raw, 256), 256, 0, stream_>>>((uint32_t)moving_, c_kind_.ptr, c_verts_.ptr,
                                                                         &sd->n_contacts, inc_off_.ptr, inc_cursor_.ptr,
-                                                                        inc_raw_.ptr);
-        k_incidence_rows<<<grid_for(8 * moving_, 128), 128, 0, stream_>>>((uint32_t)moving_, inc_off_.ptr, inc_raw_.ptr,
+                                                                        inc_raw_);
+        k_incidence_rows<<<grid_for(8 * moving_, 128), 128, 0, stream_>>>((uint32_t)moving_, inc_off_.ptr, inc_raw_,
                                                                           c_kind_.ptr, c_verts_.ptr, c_eps_.ptr,
-                                                                          inc_.ptr, inc_ref_.ptr, inc_eps_.ptr);
+                                                                          inc_, inc_ref_, inc_eps_);
         launches_ += 2;
     }
     if (moving_ > 0)
@@ -1600,7 +1604,7 @@ void World::download(std::vector<uint32_t>& kind, std::vector<uint32_t>& verts, 
     CC_CUDA(cudaMemcpy(off.data(), inc_off_.ptr, (moving_ + 1) * 4, cudaMemcpyDeviceToHost));
     inc_off.assign(off.begin(), off.end());
     inc.resize(off[moving_]);
-    if (!inc.empty()) CC_CUDA(cudaMemcpy(inc.data(), inc_.ptr, inc.size() * 4, cudaMemcpyDeviceToHost));
+    if (!inc.empty()) CC_CUDA(cudaMemcpy(inc.data(), inc_, inc.size() * 4, cudaMemcpyDeviceToHost));
     for (size_t v = 0; v < moving_; ++v) std::sort(inc.begin() + off[v], inc.begin() + off[v + 1]);
     radii.resize(moving_);
     if (moving_) CC_CUDA(cudaMemcpy(radii.data(), radii_.ptr, moving_ * 8, cudaMemcpyDeviceToHost));

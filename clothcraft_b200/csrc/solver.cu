@@ -445,11 +445,8 @@ struct cc_solver {
     DBuf<uint32_t> inc_off, inc, lo_off, lo;
     DBuf<uint2> inc_mid;  // per vertex: first hinge entry, first stitch entry
     // per-vertex records of the elastic terms (VertexTerms)
-    DBuf<uint4> vt_head;
-    DBuf<uint32_t> vt_nb;
-    DBuf<unsigned long long> vt_tri;
-    DBuf<double4> vt_tri_b, vt_tri_k;
-    DBuf<ulonglong2> vt_hinge;
+    DBuf<double4> vt_buf;  // one allocation
+    VertexTerms vt{};
     DBuf<uint4> vt_heads;  // in colour order, of the last colouring
     DBuf<uint8_t> pinned;
     DBuf<double> masses;
@@ -549,7 +546,7 @@ struct cc_solver {
         v.st_v = st_v.ptr;
         v.st_w = st_w.ptr;
         v.st_k = st_k.ptr;
-        v.vt = {vt_head.ptr, vt_nb.ptr, vt_tri.ptr, vt_tri_b.ptr, vt_tri_k.ptr, vt_hinge.ptr};
+        v.vt = vt;
         v.contacts = cv;
         v.contact_r = s.contact.radius;
         v.contact_k = s.contact.stiffness;
@@ -1415,16 +1412,21 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
         h->inc_off.upload(io, st);
         h->inc_mid.upload(mid, st);
         h->inc.upload(iv, st);
-        h->vt_head.upload(head, st);
-        h->vt_nb.upload(nb, st);
-        h->vt_tri.reserve(n_vt_tri);
-        h->vt_tri_b.reserve(n_vt_tri);
-        h->vt_tri_k.reserve(n_vt_tri);
-        h->vt_hinge.reserve(n_vt_hinge);
         {
-            const cc_vbd_settings none{};
-            launch_vertex_terms(h->sweep_view(h->world->contacts(), none, nullptr), h->vt_tri.ptr, h->vt_tri_b.ptr,
-                                h->vt_tri_k.ptr, h->vt_hinge.ptr, st);
+            // head (2 x 16 bytes a vertex), tri_b, tri_k (32), hinge (16), tri (8), nb (4) in one allocation
+            const size_t t = n_vt_tri;
+            h->vt_buf.reserve(n + 2 * t + (16 * (size_t)n_vt_hinge + 8 * t + 4 * nb.size() + 31) / 32);
+            uint4* head_d = reinterpret_cast<uint4*>(h->vt_buf.ptr);
+            double4* tri_b = h->vt_buf.ptr + n;
+            double4* tri_k = tri_b + t;
+            ulonglong2* hinge = reinterpret_cast<ulonglong2*>(tri_k + t);
+            unsigned long long* tri = reinterpret_cast<unsigned long long*>(hinge + n_vt_hinge);
+            uint32_t* nb_d = reinterpret_cast<uint32_t*>(tri + t);
+            h->vt = {head_d, nb_d, tri, tri_b, tri_k, hinge};
+            if (n) CC_CUDA(cudaMemcpyAsync(head_d, head.data(), 2 * n * sizeof(uint4), cudaMemcpyHostToDevice, st));
+            if (!nb.empty()) CC_CUDA(cudaMemcpyAsync(nb_d, nb.data(), 4 * nb.size(), cudaMemcpyHostToDevice, st));
+            launch_vertex_terms(h->sweep_view(h->world->contacts(), cc_vbd_settings{}, nullptr), tri, tri_b, tri_k,
+                                hinge, st);
         }
         h->lo_off.upload(lo_o, st);
         h->lo.upload(lo_v, st);

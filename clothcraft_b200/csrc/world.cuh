@@ -232,9 +232,13 @@ class World {
     DBuf<unsigned long long> dist_bits_;
     DBuf<double> radii_;
     DBuf<double4> centers_;
-    DBuf<uint32_t> inc_count_, inc_off_, inc_, inc_raw_, inc_cursor_;
-    DBuf<uint4> inc_ref_;
-    DBuf<double> inc_eps_;
+    DBuf<uint32_t> inc_count_, inc_off_, inc_cursor_;
+    // per incidence: the record as the row's vertex sees it, its epsilon, the
+    // contact id, and the id as the rows were dealt; one allocation
+    DBuf<uint4> inc_buf_;
+    uint4* inc_ref_ = nullptr;
+    double* inc_eps_ = nullptr;
+    uint32_t *inc_ = nullptr, *inc_raw_ = nullptr;
     RadixSorter sorter_;
     DBuf<uint32_t> scan_tmp_;
     DBuf<DetectStats> stats_d_;
