@@ -8,6 +8,7 @@
 #include <cstring>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/clothcraft.h"
@@ -163,6 +164,23 @@ inline void allow_dynamic_smem_once(K* kernel, size_t bytes, std::atomic<uint64_
     if (bit && (raised.load(std::memory_order_acquire) & bit)) return;
     allow_dynamic_smem(kernel, bytes);
     if (bit) raised.fetch_or(bit, std::memory_order_acq_rel);
+}
+
+// Launches a kernel that may start while the launch before it in the stream
+// drains (programmatic dependent launch); the kernel waits for that launch
+// itself (griddepcontrol.wait) before it reads what it wrote.
+template <class... P, class... A>
+inline void launch_after(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.stream = st;
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = a;
+    c.numAttrs = 1;
+    CC_CUDA(cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...));
 }
 
 inline int grid_for(size_t n, int block) {

@@ -292,6 +292,27 @@ __global__ void __launch_bounds__(256) k_residual_rule(StepScalars* sc, const do
     }
 }
 
+// Scalars of a batch of iterations (from iteration it0, after a detection) in
+// one launch: no refresh, stop or stall yet, a new Chebyshev sequence, clipped
+// counts and sweep-span stamps (null: off) from it0 on empty.
+__global__ void __launch_bounds__(256) k_batch_begin(StepScalars* sc, uint32_t it0, uint32_t iterations,
+                                                     unsigned long long* stamp_s, unsigned long long* stamp_e) {
+    for (uint32_t it = it0 + threadIdx.x; it < iterations; it += 256) {
+        sc->clipped_iter[it] = 0u;
+        if (stamp_s) {
+            stamp_s[it] = ~0ull;
+            stamp_e[it] = 0ull;
+        }
+    }
+    if (threadIdx.x == 0) {
+        sc->acc_k = 0u;
+        sc->acc_g2 = 1e306;
+        sc->refresh_at = sc->converged_at = sc->stop_at = 0xffffffffu;
+        sc->stall_best = 1e306;
+        sc->stall_count = 0u;
+    }
+}
+
 // Sum of the partials into *out (one block of 256 threads).
 __global__ void __launch_bounds__(256) k_store_sum(const double* partial, double* out) {
     double v = block_sum_partials(partial);
@@ -607,7 +628,8 @@ struct cc_solver {
     // full chunks after it have different shapes, and each keeps its own
     // executable, updated in place while its shape holds
     std::vector<std::pair<size_t, cudaGraphExec_t>> graph_cache;
-    static constexpr size_t kGraphCacheSize = 6;
+    static constexpr size_t kGraphCacheSize = 12;
+    uint32_t last_batch_iterations = 200;  // of the last batch of the last step: how far the next one is enqueued ahead
     uint64_t graph_instantiations = 0, graph_updates = 0;
     void launch_captured_chunk() {
         cudaGraph_t g = nullptr;
@@ -947,21 +969,12 @@ void cc_solver::step(const cc_vbd_settings& s, const cc_grab* grab, cc_metrics* 
         // the Chebyshev sequence restarts with every batch (the step's start or a refresh)
         double4* acc_prev1 = acc_a.ptr;
         double4* acc_prev2 = acc_b.ptr;
-        if (accelerate) {
+        if (accelerate)
             CC_CUDA(cudaMemcpyAsync(acc_prev1, world->x(), n * sizeof(double4), cudaMemcpyDeviceToDevice, stream));
-            CC_CUDA(cudaMemsetAsync(&sc.ptr->acc_k, 0, sizeof(unsigned int), stream));
-            CC_CUDA(cudaMemsetAsync(&sc.ptr->acc_g2, 0x7f, sizeof(double), stream));  // ~1.4e306
-        }
-        CC_CUDA(cudaMemsetAsync(&sc.ptr->refresh_at, 0xff, 2 * sizeof(unsigned int), stream));  // + converged_at
-        CC_CUDA(cudaMemsetAsync(&sc.ptr->stall_best, 0x7f, sizeof(double), stream));  // ~1.4e306
-        CC_CUDA(cudaMemsetAsync(&sc.ptr->stall_count, 0, sizeof(unsigned int), stream));
-        CC_CUDA(cudaMemsetAsync(&sc.ptr->stop_at, 0xff, sizeof(unsigned int), stream));
-        CC_CUDA(cudaMemsetAsync(&sc.ptr->clipped_iter[it0], 0, (s.iterations - it0) * sizeof(unsigned int), stream));
+        k_batch_begin<<<1, 256, 0, stream>>>(sc.ptr, it0, s.iterations, profiling ? stamp_s.ptr : nullptr,
+                                             profiling ? stamp_e.ptr : nullptr);
+        ++own_launches;
         const auto& off = coloring.offsets();
-        if (profiling) {  // this batch's iterations are (re)timed from scratch
-            CC_CUDA(cudaMemsetAsync(stamp_s.ptr + it0, 0xff, (s.iterations - it0) * sizeof(unsigned long long), stream));
-            CC_CUDA(cudaMemsetAsync(stamp_e.ptr + it0, 0, (s.iterations - it0) * sizeof(unsigned long long), stream));
-        }
         uint32_t first_color = 0, last_color = 0;
         {
             bool any = false;
@@ -972,24 +985,38 @@ void cc_solver::step(const cc_vbd_settings& s, const cc_grab* grab, cc_metrics* 
                     any = true;
                 }
         }
-        const uint32_t chunk = target_on ? std::max<uint32_t>(check_every, 4) : s.iterations;
-        uint32_t chunks = 0;
-        // graph mode: each chunk's launches (after a batch's first iteration)
-        // are captured into a CUDA graph; the executable graph of the chunk's
-        // shape is updated in place, and a new shape (another colour count or
-        // placement of the residual checks) is instantiated once and kept
+        // Iterations go out in chunks, and the host reads a chunk's stop word
+        // while the next chunk runs, so that at most one chunk is enqueued past
+        // a stop or a refresh. In graph mode a chunk's launches are captured
+        // into a CUDA graph (executables kept per shape and updated in place),
+        // except the batch's first iteration, which goes out as direct launches:
+        // the GPU starts on it while the host captures. Without a target a
+        // batch is 1 direct iteration with the next 4, then 8 at a time and what
+        // is left in powers of two: a few shapes that recur, each captured while
+        // the chunk before it runs (a single chunk of all iterations left the GPU
+        // idle for its capture and was another shape after every refresh). Where
+        // the last batch ended after its first iteration, as every one does while
+        // seams pull a garment together, the first iteration's stop word is read
+        // before anything else is enqueued.
         const bool capture = graphs;
-        for (uint32_t c0 = it0; c0 < s.iterations; c0 += chunk) {
-            uint32_t c1 = std::min(s.iterations, c0 + chunk);
-            // the batch's first iteration goes out as direct launches: the GPU
-            // starts on it while the host captures the rest of the lead chunk
-            // (the capture and the executable-graph update of the first chunk
-            // after a detection would otherwise leave the GPU idle)
-            const uint32_t cap_from = (capture && c0 == it0) ? c0 + 1 : c0;
+        const bool cautious = last_batch_iterations <= 1;
+        const uint32_t chunk = std::max<uint32_t>(check_every, 4);
+        auto power = [](uint32_t left, uint32_t most) {
+            while (most > left) most >>= 1;
+            return most;
+        };
+        uint32_t chunks = 0;
+        for (uint32_t c0 = it0, c1; c0 < s.iterations; c0 = c1) {
+            const uint32_t left = s.iterations - c0;
+            if (c0 == it0 && cautious) c1 = c0 + 1;
+            else if (target_on) c1 = c0 + std::min(left, chunk);
+            else if (c0 == it0) c1 = c0 + 1 + (left > 1 ? power(left - 1, 4) : 0);
+            else c1 = c0 + power(left, 8);
+            const uint32_t cap_from = !capture || c1 - c0 == 1 ? c1 : (c0 == it0 ? c0 + 1 : c0);
             bool capturing = false;
             try {
             for (uint32_t it = c0; it < c1; ++it) {
-                if (capture && it == cap_from) {
+                if (it == cap_from) {
                     CC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed));
                     capturing = true;
                 }
@@ -1033,13 +1060,16 @@ void cc_solver::step(const cc_vbd_settings& s, const cc_grab* grab, cc_metrics* 
             }
             if (capturing) launch_captured_chunk();
             CC_CUDA(cudaGetLastError());
-            if (c1 >= s.iterations || !target_on) break;
-            // look ahead: enqueue the next chunk before waiting on this one's stop flag
+            if (c1 >= s.iterations) break;
+            // this chunk's stop word; the last one's decides whether to go on
             unsigned int slot = chunks & 1u;
             CC_CUDA(cudaMemcpyAsync(stop_h.ptr + slot, &sc.ptr->stop_at, sizeof(unsigned int),
                                     cudaMemcpyDeviceToHost, stream));
             CC_CUDA(cudaEventRecord(chunk_ev[slot], stream));
-            if (chunks > 0) {
+            if (c0 == it0 && cautious) {
+                CC_CUDA(cudaEventSynchronize(chunk_ev[slot]));
+                if (stop_h.ptr[slot] != 0xffffffffu) break;
+            } else if (chunks > 0) {
                 CC_CUDA(cudaEventSynchronize(chunk_ev[slot ^ 1u]));
                 if (stop_h.ptr[slot ^ 1u] != 0xffffffffu) break;
             }
@@ -1048,6 +1078,7 @@ void cc_solver::step(const cc_vbd_settings& s, const cc_grab* grab, cc_metrics* 
         read_scalars();
         uint32_t ra = sc_h.ptr->refresh_at, ca = sc_h.ptr->converged_at;
         uint32_t done_to = std::min(std::min(ra, ca), s.iterations);
+        last_batch_iterations = done_to - it0;
         m.sweep_launches += (uint64_t)(done_to - it0) * coloring.n_colors();
         if (ca <= s.iterations && ca <= ra) {
             executed = ca;

@@ -23,22 +23,44 @@
 
 namespace cc {
 
+// Programmatic dependent launch: a sweep launch may start while the launch
+// before it drains. wait_for_last_launch returns once that launch is complete
+// and its writes are visible; only then does the block let the next launch
+// start, so whatever runs before the wait can rely on every launch but the last.
+__device__ __forceinline__ void wait_for_last_launch() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Solves vertex i of the colour; `wait`: the group's first vertex of the launch.
+// False if the launch is to be skipped.
 template <int G>
-__device__ __forceinline__ void solve_vertex(const SweepView& s, uint32_t i, uint32_t lane, unsigned mask, double* smem) {
+__device__ __forceinline__ bool solve_vertex(const SweepView& s, uint32_t i, uint32_t lane, unsigned mask, double* smem,
+                                             bool wait) {
     Near<G> T;
     T.head_of_color(s, i);
     const uint32_t v = T.v;
-    if (T.nt == kPinnedHead) {
-        if (lane == 0) s.residual[v] = 0.0;
-        return;
-    }
+    const bool pinned = T.nt == kPinnedHead;
+    if (pinned) T.n_nb = T.nt = T.ne = T.nw = 0u;
     // everything that the vertex's number leads to, before the first of it is waited for
-    const d3 x = ld3(s.x, v);
     const d3 y = ld3(s.target, v);
     const double m = s.inertia[v];
     const d3 ctr = ld3(s.contacts.centers, v);
     const double rad = s.contacts.radii[v];
-    const typename Near<G>::First f = T.load(s, lane, mask, smem);
+    typename Near<G>::Ids ids = T.ids(s, lane);
+    const typename Near<G>::First f = T.first(s, lane);
+    if (wait) {
+        // up to here only what earlier launches than the last one wrote; now the positions
+        wait_for_last_launch();
+        if (s.skip_at && *s.skip_at <= s.iteration) return false;  // a refresh detection precedes this iteration
+        stamp_block_start(s);
+    }
+    if (pinned) {
+        if (lane == 0) s.residual[v] = 0.0;
+        return true;
+    }
+    const d3 x = ld3(s.x, v);
+    T.stage(s, ids, lane, mask, smem);
     d3 g = mk(0, 0, 0);
     Sym H;
     sym_zero(H);
@@ -101,6 +123,7 @@ __device__ __forceinline__ void solve_vertex(const SweepView& s, uint32_t i, uin
         s.clipped_flag[v] = truncated ? 1 : 0;
         if (truncated) atomicAdd(s.clipped, 1u);
     }
+    return true;
 }
 
 // MINB blocks of BLOCK threads per SM caps the registers (65536 / (MINB*BLOCK)).
@@ -110,13 +133,14 @@ template <int G, int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB) k_sweep(SweepView s, uint32_t count) {
     constexpr uint32_t kGroups = BLOCK / G;
     __shared__ double near_s[kGroups * Near<G>::kDoubles];
-    if (s.skip_at && *s.skip_at <= s.iteration) return;  // a refresh detection precedes this iteration
     const uint32_t lane = threadIdx.x & (G - 1);
     const unsigned mask = G >= 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1)));
-    stamp_block_start(s);
-    // whole groups step together
-    for (uint32_t gi = blockIdx.x * kGroups + threadIdx.x / G; gi < count; gi += gridDim.x * kGroups)
-        solve_vertex<G>(s, gi, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
+    // whole groups step together; a grid has no more blocks than the colour needs, so a block's first group has a vertex
+    bool wait = true;
+    for (uint32_t gi = blockIdx.x * kGroups + threadIdx.x / G; gi < count; gi += gridDim.x * kGroups) {
+        if (!solve_vertex<G>(s, gi, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles, wait)) return;
+        wait = false;
+    }
     stamp_block_end(s);
 }
 
@@ -125,7 +149,7 @@ static void launch_k(const SweepView& s, uint32_t count, cudaStream_t st, unsign
     uint64_t threads = (uint64_t)count * G;
     unsigned grid = (unsigned)((threads + B - 1) / B);
     if (cap && grid > cap) grid = cap;
-    k_sweep<G, B, MINB><<<grid, B, 0, st>>>(s, count);
+    launch_after(k_sweep<G, B, MINB>, grid, B, st, s, count);
 }
 
 template <int G, int B, int MINB>

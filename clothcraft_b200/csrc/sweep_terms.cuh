@@ -410,23 +410,29 @@ struct Near {
         contact(s, c0 + lane, f);
         return f;
     }
-    // The first records, and the neighbours' positions into shared memory; the
-    // whole group calls it.
-    __device__ __forceinline__ First load(const SweepView& s, uint32_t lane, unsigned mask, double* smem) {
-        at = smem;
-        constexpr int J = (kSlots + G - 1) / G;
+    // The lane's neighbours, and their positions into shared memory (the whole
+    // group calls it).
+    static constexpr int kPer = (kSlots + G - 1) / G;
+    struct Ids {
+        uint32_t id[kPer];
+    };
+    __device__ __forceinline__ Ids ids(const SweepView& s, uint32_t lane) const {
+        Ids r;
         const uint32_t m = min(n_nb, kSlots);
-        uint32_t id[J];
-        d3 q[J];
 #pragma unroll
-        for (int j = 0; j < J; ++j) id[j] = lane + j * G < m ? s.vt.nb[nb0 + lane + j * G] : 0u;
-        const First f = first(s, lane);
+        for (int j = 0; j < kPer; ++j) r.id[j] = lane + j * G < m ? s.vt.nb[nb0 + lane + j * G] : 0u;
+        return r;
+    }
+    __device__ __forceinline__ void stage(const SweepView& s, const Ids& r, uint32_t lane, unsigned mask, double* smem) {
+        at = smem;
+        const uint32_t m = min(n_nb, kSlots);
+        d3 q[kPer];
 #pragma unroll
-        for (int j = 0; j < J; ++j)
-            if (lane + j * G < m) q[j] = ld3(s.x, id[j]);
+        for (int j = 0; j < kPer; ++j)
+            if (lane + j * G < m) q[j] = ld3(s.x, r.id[j]);
         __syncwarp(mask);  // the column's last reads are done
 #pragma unroll
-        for (int j = 0; j < J; ++j) {
+        for (int j = 0; j < kPer; ++j) {
             const uint32_t k = lane + j * G;
             if (k < m) {
                 at[k] = q[j].x;
@@ -435,6 +441,11 @@ struct Near {
             }
         }
         __syncwarp(mask);
+    }
+    __device__ __forceinline__ First load(const SweepView& s, uint32_t lane, unsigned mask, double* smem) {
+        const Ids r = ids(s, lane);
+        const First f = first(s, lane);
+        stage(s, r, lane, mask, smem);
         return f;
     }
     __device__ __forceinline__ d3 pos(const SweepView& s, uint32_t i) const {
