@@ -222,6 +222,14 @@ __global__ void k_karras(const unsigned long long* code, int m, LNode* node, int
     }
 }
 
+__global__ void k_leaf_records(const uint2* edges, const uint3* tri, const uint32_t* leaf_prim, int m, uint4* leaf) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+        const uint32_t id = leaf_prim[i];
+        if (edges) leaf[i] = make_uint4(edges[id].x, edges[id].y, edges[id].y, id);
+        else leaf[i] = make_uint4(tri[id].x, tri[id].y, tri[id].z, id);
+    }
+}
+
 __global__ void k_leaf_boxes(const Box* prim_box, const uint32_t* leaf_prim, int m, Box* leaf_box) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
         leaf_box[i] = prim_box[leaf_prim[i]];
@@ -276,7 +284,8 @@ __global__ void k_lbvh_refit(const Box* leaf_box, const uint32_t* leaf_prim, int
     }
 }
 
-int Lbvh::build(const Box* prim_box, const uint32_t* ids, uint32_t count, cudaStream_t s, unsigned int* err) {
+int Lbvh::build(const Box* prim_box, const uint32_t* ids, uint32_t count, const uint2* edges, const uint3* tri,
+                cudaStream_t s, unsigned int* err) {
     m = count;
     built = true;
     if (m == 0) return 0;
@@ -289,11 +298,13 @@ int Lbvh::build(const Box* prim_box, const uint32_t* ids, uint32_t count, cudaSt
     parent.reserve(2 * m);
     visits.reserve(m);
     leaf_box.reserve(m);
+    leaf.reserve(m);
     k_bounds_init<<<1, 32, 0, s>>>(bounds.ptr);
     k_centroid_bounds<<<grid_for(m, 256), 256, 0, s>>>(prim_box, ids, m, bounds.ptr);
     k_morton<<<grid_for(m, 256), 256, 0, s>>>(prim_box, ids, m, bounds.ptr, morton_tmp.ptr, ids_tmp.ptr);
     int sorts = sorter.sort_pairs(morton_tmp.ptr, morton.ptr, ids_tmp.ptr, leaf_prim.ptr, m, 63, s, err, DERR_SORT_WAIT);
-    int n = 3 + sorts;
+    k_leaf_records<<<grid_for(m, 256), 256, 0, s>>>(edges, tri, leaf_prim.ptr, (int)m, leaf.ptr);
+    int n = 4 + sorts;
     if (m > 1) {
         k_karras<<<grid_for(m - 1, 256), 256, 0, s>>>(morton.ptr, (int)m, node.ptr, parent.ptr);
         ++n;
@@ -351,8 +362,8 @@ __device__ __forceinline__ bool overlap32(const QBox& q, float lx, float ly, flo
 
 // Depth-first traversal that goes down one passing child and stacks the
 // other. near(lx, ly, lz, hx, hy, hz) tests a child's FP32 box; leaf_ok(box)
-// is the exact FP64 primitive predicate; visit(prim) receives the accepted
-// primitive id. With ABOVE, only primitives with id > above are visited and
+// is the exact FP64 primitive predicate; visit(leaf record) receives the accepted
+// primitives. With ABOVE, only primitives with id > above are visited and
 // subtrees whose largest id is <= above are skipped unvisited (self-pair
 // queries that keep the canonical order e < f). Returns false if the stack
 // overflowed.
@@ -361,8 +372,8 @@ template <bool ABOVE, class Near, class LeafOk, class Visit>
 __device__ __forceinline__ bool lbvh_walk(const LbvhView& t, uint32_t above, Near near, LeafOk leaf_ok, Visit visit) {
     if (t.m == 0) return true;
     if (t.m == 1) {
-        uint32_t p = t.leaf_prim[0];
-        if ((!ABOVE || p > above) && leaf_ok(t.leaf_box[0])) visit(p);
+        const uint4 p = t.leaf[0];
+        if ((!ABOVE || p.w > above) && leaf_ok(t.leaf_box[0])) visit(p);
         return true;
     }
     int stack[kTraversalStack];
@@ -376,12 +387,14 @@ __device__ __forceinline__ bool lbvh_walk(const LbvhView& t, uint32_t above, Nea
         bool go_r = (!ABOVE || (uint32_t)d.w > above) && near(b.z, b.w, c.x, c.y, c.z, c.w);
         if (go_l && d.x < 0) {
             uint32_t i = (uint32_t)d.x & 0x7fffffffu;
-            if (leaf_ok(t.leaf_box[i])) visit(t.leaf_prim[i]);
+            const uint4 p = __ldg(t.leaf + i);
+            if (leaf_ok(t.leaf_box[i])) visit(p);
             go_l = false;
         }
         if (go_r && d.y < 0) {
             uint32_t i = (uint32_t)d.y & 0x7fffffffu;
-            if (leaf_ok(t.leaf_box[i])) visit(t.leaf_prim[i]);
+            const uint4 p = __ldg(t.leaf + i);
+            if (leaf_ok(t.leaf_box[i])) visit(p);
             go_r = false;
         }
         if (go_l && go_r) {
@@ -613,71 +626,109 @@ __device__ __forceinline__ unsigned long long append_slot(unsigned long long* co
     return g.shfl(base, 0) + g.thread_rank();
 }
 
+// Pairs of one query, gathered in the thread's column of shared memory and
+// appended to the list 16 at a time: one atomic with its round trip per 16 pairs
+// instead of one per accepted leaf, and runs of one query in the list, whose
+// gathers the narrow phase's neighbouring lanes share.
+constexpr int kQueryBlock = 128;
+constexpr uint32_t kPairBuffer = 16;
+struct PairSink {
+    uint32_t* column;  // [kPairBuffer] at stride kQueryBlock
+    uint2* out;
+    unsigned long long cap;
+    unsigned long long* count;
+    uint32_t query, n;
+    __device__ __forceinline__ void flush() {
+        if (n == 0) return;
+        const unsigned long long base = atomicAdd(count, (unsigned long long)n);
+        for (uint32_t i = 0; i < n; ++i)
+            if (base + i < cap) out[base + i] = make_uint2(query, column[i * kQueryBlock]);
+        n = 0;
+    }
+    __device__ __forceinline__ void push(uint32_t id) {
+        column[n * kQueryBlock] = id;
+        if (++n == kPairBuffer) flush();
+    }
+};
+
+// The excluded neighbours of a query's vertex, looked up once: nearly all have none.
+struct Excluded {
+    uint32_t v, lo, hi;
+    __device__ __forceinline__ Excluded(const WorldView& w, uint32_t vertex)
+        : v(vertex), lo(w.ex_off[vertex]), hi(w.ex_off[vertex + 1]) {}
+    __device__ __forceinline__ bool adjacent_to(const WorldView& w, uint32_t b) const {  // world.rs:215-217
+        if (v == b) return true;
+        uint32_t l = lo, h = hi;
+        while (l < h) {
+            const uint32_t mid = (l + h) >> 1, x = w.ex[mid];
+            if (x == b) return true;
+            if (x < b) l = mid + 1;
+            else h = mid;
+        }
+        return false;
+    }
+};
+
 // VF candidates (candidates.rs:29-37): every point against triangles, pairs
 // with box distance <= search, not both fixed, triangle not adjacent.
 // Points are taken in `order` (a Morton order of the points), so that the
 // lanes of a warp walk nearby points. (Walking a warp's 32 queries as one
 // node sequence, the union of their walks, measured 4x slower for VF and
 // 1.2x for EE on the fold: the union is several times the longest walk.)
-__global__ void k_vf_query(WorldView w, const uint32_t* order, LbvhView tri_moving, LbvhView tri_fixed, double search2,
-                           uint2* out, unsigned long long cap, unsigned long long* count, unsigned int* err) {
+__global__ void __launch_bounds__(kQueryBlock) k_vf_query(WorldView w, const uint32_t* order, LbvhView tri_moving,
+                                                          LbvhView tri_fixed, double search2, uint2* out,
+                                                          unsigned long long cap, unsigned long long* count,
+                                                          unsigned int* err) {
+    __shared__ uint32_t buffer[kPairBuffer * kQueryBlock];
     const float r2 = r2_bound(search2);
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < w.n_all; j += gridDim.x * blockDim.x) {
+    for (uint32_t j = blockIdx.x * kQueryBlock + threadIdx.x; j < w.n_all; j += gridDim.x * kQueryBlock) {
         const uint32_t v = order[j];
+        const Excluded ex(w, v);
         Box q;
         box_of1(ld3(w.x, v), q);
         const QBox q32 = qbox(q);
+        PairSink sink{buffer + threadIdx.x, out, cap, count, v, 0u};
         auto near = [&](float lx, float ly, float lz, float hx, float hy, float hz) {
             return near32(q32, lx, ly, lz, hx, hy, hz, r2);
         };
         auto leaf_ok = [&](const Box& b) { return box_dist2(q, b) <= search2; };
-        auto visit = [&](uint32_t t) {
-            uint3 ids = w.tri[t];
-            if (adjacent(w, v, ids.x) || adjacent(w, v, ids.y) || adjacent(w, v, ids.z)) return;
-            unsigned long long k = append_slot(count);
-            if (k < cap) out[k] = make_uint2(v, t);
+        auto visit = [&](uint4 t) {
+            if (!(ex.adjacent_to(w, t.x) || ex.adjacent_to(w, t.y) || ex.adjacent_to(w, t.z))) sink.push(t.w);
         };
         bool ok = lbvh_walk<false>(tri_moving, 0u, near, leaf_ok, visit);
         if (v < w.moving) ok = lbvh_walk<false>(tri_fixed, 0u, near, leaf_ok, visit) && ok;
+        sink.flush();
         if (!ok) atomicOr(err, DERR_STACK_OVERFLOW);
     }
 }
 
 // EE candidates (candidates.rs:38-55): moving edges against moving edges
 // (each unordered pair once, canonical e < f) and against fixed edges
-// (moving edge first). `edge_moving` lists the moving edges in the moving
-// edge tree's leaf order (a Morton order), so neighbouring lanes query
-// neighbouring edges.
-__global__ void k_ee_query(WorldView w, const uint32_t* edge_moving, uint32_t n_moving_edges, LbvhView edge_moving_t,
-                           LbvhView edge_fixed_t, double search2, uint2* out, unsigned long long cap,
-                           unsigned long long* count, unsigned int* err) {
+// (moving edge first). The moving edges are taken in the moving edge tree's
+// leaf order (a Morton order), so neighbouring lanes query neighbouring edges.
+__global__ void __launch_bounds__(kQueryBlock) k_ee_query(WorldView w, LbvhView edge_moving_t, LbvhView edge_fixed_t,
+                                                          double search2, uint2* out, unsigned long long cap,
+                                                          unsigned long long* count, unsigned int* err) {
+    __shared__ uint32_t buffer[kPairBuffer * kQueryBlock];
     const float r2 = r2_bound(search2);
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_moving_edges; k += gridDim.x * blockDim.x) {
-        uint32_t e = edge_moving[k];
-        Box q = w.edge_box[e];
+    for (uint32_t k = blockIdx.x * kQueryBlock + threadIdx.x; k < edge_moving_t.m; k += gridDim.x * kQueryBlock) {
+        const uint4 e = edge_moving_t.leaf[k];
+        const Box q = edge_moving_t.leaf_box[k];
         const QBox q32 = qbox(q);
-        uint2 ids = w.edges[e];
+        const Excluded ex0(w, e.x), ex1(w, e.y);
+        PairSink sink{buffer + threadIdx.x, out, cap, count, e.w, 0u};
         auto near = [&](float lx, float ly, float lz, float hx, float hy, float hz) {
             return near32(q32, lx, ly, lz, hx, hy, hz, r2);
         };
         auto leaf_ok = [&](const Box& b) { return box_dist2(q, b) <= search2; };
-        auto filtered = [&](uint32_t f) {
-            uint2 js = w.edges[f];
-            return adjacent(w, ids.x, js.x) || adjacent(w, ids.x, js.y) || adjacent(w, ids.y, js.x) ||
-                   adjacent(w, ids.y, js.y);
+        auto visit = [&](uint4 f) {  // f.w > e.w for moving edges: the walk leaves the others out
+            if (!(ex0.adjacent_to(w, f.x) || ex0.adjacent_to(w, f.y) || ex1.adjacent_to(w, f.x) ||
+                  ex1.adjacent_to(w, f.y)))
+                sink.push(f.w);
         };
-        auto visit_moving = [&](uint32_t f) {
-            if (f <= e || filtered(f)) return;
-            unsigned long long i = append_slot(count);
-            if (i < cap) out[i] = make_uint2(e, f);
-        };
-        auto visit_fixed = [&](uint32_t f) {
-            if (filtered(f)) return;
-            unsigned long long i = append_slot(count);
-            if (i < cap) out[i] = make_uint2(e, f);
-        };
-        bool ok = lbvh_walk<true>(edge_moving_t, e, near, leaf_ok, visit_moving);
-        ok = lbvh_walk<false>(edge_fixed_t, 0u, near, leaf_ok, visit_fixed) && ok;
+        bool ok = lbvh_walk<true>(edge_moving_t, e.w, near, leaf_ok, visit);
+        ok = lbvh_walk<false>(edge_fixed_t, 0u, near, leaf_ok, visit) && ok;
+        sink.flush();
         if (!ok) atomicOr(err, DERR_STACK_OVERFLOW);
     }
 }
@@ -994,8 +1045,9 @@ __global__ void k_intersections(WorldView w, LbvhView tri_moving, LbvhView tri_f
             q.hi[k] = q.hi[k] + 1e-10;
         }
         uint32_t tv[3] = {t.x, t.y, t.z};
-        auto visit = [&](uint32_t j) {
-            uint3 qq = w.tri[j];
+        auto visit = [&](uint4 rec) {
+            const uint32_t j = rec.w;
+            const uint3 qq = make_uint3(rec.x, rec.y, rec.z);
             bool q_fixed = qq.x >= w.moving && qq.y >= w.moving && qq.z >= w.moving;
             if (j <= i || (t_fixed && q_fixed)) return;
             uint32_t qv[3] = {qq.x, qq.y, qq.z};
@@ -1199,8 +1251,10 @@ World::World(const double* x_all, size_t n_all, const std::vector<std::array<uin
     // fixed trees are built once: fixed geometry never moves
     stats_d_.zero(1, stream_);
     refit(false);
-    tree_tri_fixed_.build(tri_box_.ptr, tri_fixed_.ptr, (uint32_t)tri_fixed_h_.size(), stream_, &stats_d_.ptr->error);
-    tree_edge_fixed_.build(edge_box_.ptr, edge_fixed_.ptr, (uint32_t)edge_fixed_h_.size(), stream_, &stats_d_.ptr->error);
+    tree_tri_fixed_.build(tri_box_.ptr, tri_fixed_.ptr, (uint32_t)tri_fixed_h_.size(), nullptr, tri_.ptr, stream_,
+                          &stats_d_.ptr->error);
+    tree_edge_fixed_.build(edge_box_.ptr, edge_fixed_.ptr, (uint32_t)edge_fixed_h_.size(), edges_.ptr, nullptr, stream_,
+                           &stats_d_.ptr->error);
     CC_CUDA(cudaStreamSynchronize(stream_));
 }
 
@@ -1271,9 +1325,11 @@ int World::update_trees() {
     CC_CUDA(cudaEventRecord(fork_, stream_));
     CC_CUDA(cudaStreamWaitEvent(side_, fork_, 0));
     unsigned int* err = &stats_d_.ptr->error;
-    int n = build ? tree_tri_moving_.build(tri_box_.ptr, tri_moving_.ptr, (uint32_t)tri_moving_h_.size(), side_, err)
+    int n = build ? tree_tri_moving_.build(tri_box_.ptr, tri_moving_.ptr, (uint32_t)tri_moving_h_.size(), nullptr, tri_.ptr,
+                                           side_, err)
                   : tree_tri_moving_.refit(tri_box_.ptr, side_);
-    n += build ? tree_edge_moving_.build(edge_box_.ptr, edge_moving_.ptr, (uint32_t)edge_moving_h_.size(), stream_, err)
+    n += build ? tree_edge_moving_.build(edge_box_.ptr, edge_moving_.ptr, (uint32_t)edge_moving_h_.size(), edges_.ptr, nullptr,
+                                        stream_, err)
                : tree_edge_moving_.refit(edge_box_.ptr, stream_);
     if (build) n += order_points();
     return n;
@@ -1303,7 +1359,6 @@ void World::build_candidates(double R, double skin) {
     launches_ += update_trees();
     LbvhView tm = tree_tri_moving_.view(), tf = tree_tri_fixed_.view();
     LbvhView em = tree_edge_moving_.view(), ef = tree_edge_fixed_.view();
-    const uint32_t* edges_in_leaf_order = tree_edge_moving_.leaf_prim.ptr;
     if (vf_cap_ == 0) {
         // generous first capacities: the in-plane pairs of a sheet at the
         // candidate radius alone reach ~60 per edge
@@ -1325,8 +1380,7 @@ void World::build_candidates(double R, double skin) {
         k_vf_query<<<grid_for(n_all_, 128), 128, 0, side_>>>(view(), point_order_.ptr, tm, tf, search2, vf_.ptr,
                                                               vf_cap_, &stats_d_.ptr->n_vf, &stats_d_.ptr->error);
         k_ee_query<<<grid_for(edge_moving_h_.size(), 128), 128, 0, stream_>>>(
-            view(), edges_in_leaf_order, (uint32_t)edge_moving_h_.size(), em, ef, search2, ee_.ptr, ee_cap_,
-            &stats_d_.ptr->n_ee, &stats_d_.ptr->error);
+            view(), em, ef, search2, ee_.ptr, ee_cap_, &stats_d_.ptr->n_ee, &stats_d_.ptr->error);
         launches_ += 2;
         CC_CUDA(cudaGetLastError());
         CC_CUDA(cudaEventRecord(join_, side_));
@@ -1559,8 +1613,7 @@ void World::fresh_pairs(double search, std::vector<uint32_t>& vf, std::vector<ui
         k_vf_query<<<grid_for(n_all_, 128), 128, 0, stream_>>>(view(), point_order_.ptr, tm, tf, search2, a.ptr,
                                                                 vcap, fresh_counts_.ptr, &stats_d_.ptr->error);
         k_ee_query<<<grid_for(edge_moving_h_.size(), 128), 128, 0, stream_>>>(
-            view(), tree_edge_moving_.leaf_prim.ptr, (uint32_t)edge_moving_h_.size(), em, ef, search2, b.ptr, ecap,
-            fresh_counts_.ptr + 1, &stats_d_.ptr->error);
+            view(), em, ef, search2, b.ptr, ecap, fresh_counts_.ptr + 1, &stats_d_.ptr->error);
         CC_CUDA(cudaGetLastError());
         unsigned long long counts[2];
         CC_CUDA(cudaMemcpyAsync(counts, fresh_counts_.ptr, sizeof counts, cudaMemcpyDeviceToHost, stream_));

@@ -31,7 +31,7 @@ struct alignas(16) LNode {
 struct LbvhView {
     uint32_t m;                 // leaves
     const LNode* node;          // [m-1] internal nodes, root 0
-    const uint32_t* leaf_prim;  // [m] primitive id of each sorted leaf
+    const uint4* leaf;          // [m] each sorted leaf's primitive: vertices (an edge's second one twice) and id
     const Box* leaf_box;        // [m] exact primitive boxes in leaf order
 };
 
@@ -47,14 +47,17 @@ struct Lbvh {
     DBuf<int> parent;       // [2m-1]: internal 0..m-2, leaves m-1..2m-2
     DBuf<unsigned> visits;  // [m-1]
     DBuf<uint32_t> leaf_prim, ids_tmp;
+    DBuf<uint4> leaf;       // [m]
     DBuf<Box> leaf_box;     // [m]
     DBuf<unsigned long long> morton, morton_tmp;
     DBuf<unsigned long long> bounds;  // 6 order keys
     RadixSorter sorter;
-    // Both return the number of this library's kernels launched.
-    int build(const Box* prim_box, const uint32_t* ids, uint32_t m, cudaStream_t s, unsigned int* err);
+    // Both return the number of this library's kernels launched. The primitives
+    // are `edges` or `tri`, whichever is not null.
+    int build(const Box* prim_box, const uint32_t* ids, uint32_t m, const uint2* edges, const uint3* tri, cudaStream_t s,
+              unsigned int* err);
     int refit(const Box* prim_box, cudaStream_t s);  // after a build over the same primitives
-    LbvhView view() const { return {m, node.ptr, leaf_prim.ptr, leaf_box.ptr}; }
+    LbvhView view() const { return {m, node.ptr, leaf.ptr, leaf_box.ptr}; }
 };
 
 // Static topology (src/ogc/topology.rs:13-52), built on the host at creation.
