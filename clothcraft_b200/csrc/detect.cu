@@ -502,17 +502,6 @@ __device__ d3 closest_on_triangle(d3 p, d3 a, d3 b, d3 c, int& kind, int& which)
     return a + ab * (vb * denom) + ac * (vc * denom);
 }
 
-// closest_triangle on world triangle t, returning the feature's id.
-__device__ d3 closest_triangle(const WorldView& w, d3 p, uint32_t t, int& kind, uint32_t& fid) {
-    uint3 ids = w.tri[t];
-    int which;
-    d3 q = closest_on_triangle(p, ld3(w.x, ids.x), ld3(w.x, ids.y), ld3(w.x, ids.z), kind, which);
-    if (kind == 0) fid = which == 0 ? ids.x : (which == 1 ? ids.y : ids.z);
-    else if (kind == 1) fid = which == 0 ? w.tri_edges[t].x : (which == 1 ? w.tri_edges[t].y : w.tri_edges[t].z);
-    else fid = t;
-    return q;
-}
-
 __device__ __forceinline__ double clamp01(double x) { return x < 0.0 ? 0.0 : (x > 1.0 ? 1.0 : x); }
 
 // closest_segments (geometry.rs:78-107)
@@ -779,84 +768,158 @@ __device__ __forceinline__ void push_ee(const NarrowOut& o, uint32_t e, uint2 id
     else push_key(o, 3, re, rf);
 }
 
-__global__ void k_narrow(WorldView w, const uint2* vf, unsigned long long n_vf, const uint2* ee,
-                         unsigned long long n_ee, double query_radius, const unsigned long long* max_abs_bits,
-                         int prune, NarrowOut o) {
+// One pair per lane. A pair in range whose closest feature is a vertex or, for a
+// point, an edge has to pass the feasibility tests (loops over the feature's
+// neighbours that most pairs fail early); such pairs go to the warp's queue in
+// shared memory and are tested 32 at a time, so that the tests run on full warps
+// instead of on the ~quarter of the lanes whose pair is in range. Boxes are formed
+// from the positions, which a pair that is not rejected needs anyway (min and max
+// are exact: the same boxes as k_refit's), one dependent load less than
+// reading them. Bound by those gathers (pair -> vertices -> positions).
+constexpr int kNarrowBlock = 128;
+constexpr uint32_t kNarrowQueue = 64;
+enum NarrowTest : uint32_t { TEST_VERTEX = 0, TEST_EDGE = 1, TEST_EDGES = 2 };
+struct NarrowQueue {
+    uint2 pair[kNarrowQueue];
+    uint32_t test[kNarrowQueue];
+    // a point's feature id (s), or the parameters of the closest points of two edges
+    double s[kNarrowQueue], t[kNarrowQueue];
+};
+
+__device__ __forceinline__ void narrow_test(const WorldView& w, const NarrowOut& o, const NarrowQueue& q, uint32_t i) {
+    const uint2 pr = q.pair[i];
+    if (q.test[i] != TEST_EDGES) {
+        const d3 xv = ld3(w.x, pr.x);
+        const uint32_t fid = (uint32_t)__double_as_longlong(q.s[i]);
+        if (q.test[i] == TEST_VERTEX) {
+            if (vertex_feasible(w, xv, fid)) push_pp(o, pr.x, fid);
+        } else {
+            if (edge_feasible(w, xv, fid)) push_pe(o, pr.x, fid);
+        }
+        return;
+    }
+    const double s = q.s[i], t = q.t[i];
+    const uint2 ids = w.edges[pr.x], js = w.edges[pr.y];
+    const d3 a = ld3(w.x, ids.x), b = ld3(w.x, ids.y), c = ld3(w.x, js.x), dd = ld3(w.x, js.y);
+    const d3 p = a + (b - a) * s;
+    const d3 r = c + (dd - c) * t;
+    const long end_a = s <= 0.0 ? (long)ids.x : (s >= 1.0 ? (long)ids.y : -1);
+    const long end_b = t <= 0.0 ? (long)js.x : (t >= 1.0 ? (long)js.y : -1);
+    if ((end_a >= 0 && !vertex_feasible(w, r, (uint32_t)end_a)) || (end_b >= 0 && !vertex_feasible(w, p, (uint32_t)end_b)))
+        return;
+    if (end_a >= 0 && end_b >= 0) push_pp(o, (uint32_t)end_a, (uint32_t)end_b);
+    else if (end_a >= 0) push_pe(o, (uint32_t)end_a, pr.y);
+    else push_pe(o, (uint32_t)end_b, pr.x);
+}
+
+__global__ void __launch_bounds__(kNarrowBlock) k_narrow(WorldView w, const uint2* vf, unsigned long long n_vf,
+                                                         const uint2* ee, unsigned long long n_ee, double query_radius,
+                                                         const unsigned long long* max_abs_bits, int prune, NarrowOut o) {
+    __shared__ NarrowQueue queues[kNarrowBlock / 32];
+    NarrowQueue& queue = queues[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t queued = 0;
     double scale = fmax(query_radius, bitsd(*max_abs_bits));
     double pr = query_radius + 64.0 * 2.220446049250313e-16 * scale;
     double padded2 = pr * pr;
     unsigned long long nvf = 0, nee = 0, nrej = 0;
-    unsigned long long total = n_vf + n_ee;
-    for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-         k += (unsigned long long)gridDim.x * blockDim.x) {
+    const unsigned long long total = n_vf + n_ee;
+    // whole warps step together
+    for (unsigned long long k0 = (unsigned long long)blockIdx.x * kNarrowBlock + (threadIdx.x & ~31u); k0 < total;
+         k0 += (unsigned long long)gridDim.x * kNarrowBlock) {
+        const unsigned long long k = k0 + lane;
+        bool test = false;
+        uint32_t kind_of_test = 0;
+        uint2 pair = make_uint2(0u, 0u);
+        double qs = 0.0, qt = 0.0;
         if (k < n_vf) {
-            uint32_t v = vf[k].x, t = vf[k].y;
-            d3 xv = ld3(w.x, v);
-            if (prune) {
-                Box pb;
-                box_of1(xv, pb);
-                if (box_dist2(pb, w.tri_box[t]) > padded2) {
-                    ++nrej;
-                    continue;
+            pair = vf[k];
+            const uint32_t v = pair.x, t = pair.y;
+            const uint3 ids = w.tri[t];
+            const d3 xv = ld3(w.x, v);
+            const d3 a = ld3(w.x, ids.x), b = ld3(w.x, ids.y), c = ld3(w.x, ids.z);
+            Box pb, tb;
+            box_of1(xv, pb);
+            box_of3(a, b, c, tb);
+            if (prune && box_dist2(pb, tb) > padded2) {
+                ++nrej;
+            } else {
+                int kind, which;
+                const d3 p = closest_on_triangle(xv, a, b, c, kind, which);
+                const double d = len(xv - p);
+                if (!(d >= query_radius)) {
+                    ++nvf;
+                    const unsigned long long db = dbits(d);
+                    atomicMin(&o.dist[v], db);
+                    atomicMin(&o.dist[ids.x], db);
+                    atomicMin(&o.dist[ids.y], db);
+                    atomicMin(&o.dist[ids.z], db);
+                    if (kind == 2) {
+                        push_pf(o, v, t);
+                    } else {
+                        uint32_t fid;
+                        if (kind == 0) fid = which == 0 ? ids.x : (which == 1 ? ids.y : ids.z);
+                        else fid = which == 0 ? w.tri_edges[t].x : (which == 1 ? w.tri_edges[t].y : w.tri_edges[t].z);
+                        test = true;
+                        kind_of_test = kind == 0 ? TEST_VERTEX : TEST_EDGE;
+                        qs = __longlong_as_double((long long)fid);
+                    }
                 }
             }
-            uint3 ids = w.tri[t];
-            int kind;
-            uint32_t fid;
-            d3 p = closest_triangle(w, xv, t, kind, fid);
-            double d = len(xv - p);
-            if (d >= query_radius) continue;
-            ++nvf;
-            unsigned long long db = dbits(d);
-            atomicMin(&o.dist[v], db);
-            atomicMin(&o.dist[ids.x], db);
-            atomicMin(&o.dist[ids.y], db);
-            atomicMin(&o.dist[ids.z], db);
-            if (kind == 0) {
-                if (vertex_feasible(w, xv, fid)) push_pp(o, v, fid);
-            } else if (kind == 1) {
-                if (edge_feasible(w, xv, fid)) push_pe(o, v, fid);
-            } else {
-                push_pf(o, v, t);
-            }
-        } else {
-            unsigned long long kk = k - n_vf;
-            uint32_t e = ee[kk].x, f = ee[kk].y;
-            if (prune && box_dist2(w.edge_box[e], w.edge_box[f]) > padded2) {
+        } else if (k < total) {
+            pair = ee[k - n_vf];
+            const uint2 ids = w.edges[pair.x], js = w.edges[pair.y];
+            const d3 a = ld3(w.x, ids.x), b = ld3(w.x, ids.y), c = ld3(w.x, js.x), dd = ld3(w.x, js.y);
+            Box be, bf;
+            box_of2(a, b, be);
+            box_of2(c, dd, bf);
+            if (prune && box_dist2(be, bf) > padded2) {
                 ++nrej;
-                continue;
+            } else {
+                closest_segments(a, b, c, dd, qs, qt);
+                const d3 p = a + (b - a) * qs;
+                const d3 q = c + (dd - c) * qt;
+                const double dist = len(p - q);
+                if (!(dist >= query_radius)) {
+                    ++nee;
+                    const unsigned long long db = dbits(dist);
+                    atomicMin(&o.dist[ids.x], db);
+                    atomicMin(&o.dist[ids.y], db);
+                    atomicMin(&o.dist[js.x], db);
+                    atomicMin(&o.dist[js.y], db);
+                    if (qs <= 0.0 || qs >= 1.0 || qt <= 0.0 || qt >= 1.0) {
+                        test = true;
+                        kind_of_test = TEST_EDGES;
+                    } else {
+                        push_ee(o, pair.x, ids, pair.y, js);
+                    }
+                }
             }
-            uint2 ids = w.edges[e], js = w.edges[f];
-            d3 a = ld3(w.x, ids.x), b = ld3(w.x, ids.y), c = ld3(w.x, js.x), dd = ld3(w.x, js.y);
-            double s, t;
-            closest_segments(a, b, c, dd, s, t);
-            d3 p = a + (b - a) * s;
-            d3 q = c + (dd - c) * t;
-            double dist = len(p - q);
-            if (dist >= query_radius) continue;
-            ++nee;
-            unsigned long long db = dbits(dist);
-            atomicMin(&o.dist[ids.x], db);
-            atomicMin(&o.dist[ids.y], db);
-            atomicMin(&o.dist[js.x], db);
-            atomicMin(&o.dist[js.y], db);
-            long end_a = s <= 0.0 ? (long)ids.x : (s >= 1.0 ? (long)ids.y : -1);
-            long end_b = t <= 0.0 ? (long)js.x : (t >= 1.0 ? (long)js.y : -1);
-            if ((end_a >= 0 && !vertex_feasible(w, q, (uint32_t)end_a)) ||
-                (end_b >= 0 && !vertex_feasible(w, p, (uint32_t)end_b)))
-                continue;
-            if (end_a >= 0 && end_b >= 0) push_pp(o, (uint32_t)end_a, (uint32_t)end_b);
-            else if (end_a >= 0) push_pe(o, (uint32_t)end_a, f);
-            else if (end_b >= 0) push_pe(o, (uint32_t)end_b, e);
-            else push_ee(o, e, ids, f, js);
+        }
+        __syncwarp();  // the queue's last reads are done
+        const unsigned in = __ballot_sync(0xffffffffu, test);
+        if (test) {
+            const uint32_t i = queued + __popc(in & ((1u << lane) - 1u));
+            queue.pair[i] = pair;
+            queue.test[i] = kind_of_test;
+            queue.s[i] = qs;
+            queue.t[i] = qt;
+        }
+        queued += __popc(in);  // below 32 before, at most 63 now
+        __syncwarp();
+        if (queued >= 32) {
+            queued -= 32;
+            narrow_test(w, o, queue, queued + lane);
         }
     }
+    __syncwarp();
+    if (lane < queued) narrow_test(w, o, queue, lane);
     for (int s = 16; s > 0; s >>= 1) {
         nvf += __shfl_xor_sync(0xffffffffu, nvf, s);
         nee += __shfl_xor_sync(0xffffffffu, nee, s);
         nrej += __shfl_xor_sync(0xffffffffu, nrej, s);
     }
-    if ((threadIdx.x & 31) == 0) {
+    if (lane == 0) {
         if (nvf) atomicAdd(o.vf_count, nvf);
         if (nee) atomicAdd(o.ee_count, nee);
         if (nrej) atomicAdd(o.rejections, nrej);
@@ -1470,7 +1533,7 @@ void World::detect(double query_radius, double radius, double relaxation, double
         NarrowOut o{raw_key_.ptr,    raw_cap_,           &sd->n_raw,        dist_bits_.ptr, &sd->vf_count,
                     &sd->ee_count,   &sd->rejections,    edge_rank_.ptr,    tri_rank_.ptr,  key_bits_};
         unsigned long long total = n_vf + n_ee;
-        k_narrow<<<grid_for((size_t)total, 128), 128, 0, stream_>>>(view(), vf_.ptr, n_vf, ee_.ptr, n_ee, query_radius,
+        k_narrow<<<grid_for((size_t)total, kNarrowBlock), kNarrowBlock, 0, stream_>>>(view(), vf_.ptr, n_vf, ee_.ptr, n_ee, query_radius,
                                                                     &sd->max_abs_bits, prune ? 1 : 0, o);
         launches_ += 2;
         CC_CUDA(cudaGetLastError());
