@@ -1705,25 +1705,49 @@ void World::fresh_pairs(double search, std::vector<uint32_t>& vf, std::vector<ui
     throw Failure{CC_ERR_CUDA, "OGC candidate buffers could not be sized"};
 }
 
-void World::download(std::vector<uint32_t>& kind, std::vector<uint32_t>& verts, std::vector<double>& eps,
-                     std::vector<uint64_t>& inc_off, std::vector<uint32_t>& inc, std::vector<double>& radii) {
-    size_t n = stats_h_.ptr->n_contacts;
-    kind.resize(n);
-    verts.resize(4 * n);
-    eps.resize(n);
-    if (n) {
-        CC_CUDA(cudaMemcpy(kind.data(), c_kind_.ptr, n * 4, cudaMemcpyDeviceToHost));
-        CC_CUDA(cudaMemcpy(verts.data(), c_verts_.ptr, n * 16, cudaMemcpyDeviceToHost));
-        CC_CUDA(cudaMemcpy(eps.data(), c_eps_.ptr, n * 8, cudaMemcpyDeviceToHost));
+// the parts of the contact set whose host types differ from the device's
+__global__ void k_export(size_t n, size_t moving, const uint32_t* kind, const uint32_t* off, uint64_t* off64,
+                         uint8_t* kinds, uint8_t* counts) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x, i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (size_t i = i0; i <= moving; i += stride) off64[i] = off[i];
+    for (size_t i = i0; i < n; i += stride) {
+        kinds[i] = (uint8_t)kind[i];
+        counts[i] = (uint8_t)kind_count(kind[i]);
     }
-    std::vector<uint32_t> off(moving_ + 1);
-    CC_CUDA(cudaMemcpy(off.data(), inc_off_.ptr, (moving_ + 1) * 4, cudaMemcpyDeviceToHost));
-    inc_off.assign(off.begin(), off.end());
-    inc.resize(off[moving_]);
-    if (!inc.empty()) CC_CUDA(cudaMemcpy(inc.data(), inc_, inc.size() * 4, cudaMemcpyDeviceToHost));
-    for (size_t v = 0; v < moving_; ++v) std::sort(inc.begin() + off[v], inc.begin() + off[v + 1]);
-    radii.resize(moving_);
-    if (moving_) CC_CUDA(cudaMemcpy(radii.data(), radii_.ptr, moving_ * 8, cudaMemcpyDeviceToHost));
+}
+
+World::HostContacts World::fetch() {
+    const size_t n = stats_h_.ptr->n_contacts, ni = stats_h_.ptr->n_incident, m = moving_;
+    const size_t dev = 8 * (m + 1) + 2 * n;  // offsets, kinds, counts
+    fetch_d_.reserve(dev);
+    uint64_t* off64 = reinterpret_cast<uint64_t*>(fetch_d_.ptr);
+    uint8_t* kinds = fetch_d_.ptr + 8 * (m + 1);
+    k_export<<<grid_for(std::max(n, m + 1), 256), 256, 0, stream_>>>(n, m, c_kind_.ptr, inc_off_.ptr, off64, kinds,
+                                                                     kinds + n);
+    ++launches_;
+    CC_CUDA(cudaGetLastError());
+    const size_t bytes = 16 * n + 8 * n + 8 * m + dev + 4 + 4 * ni;
+    if (bytes > fetch_h_.cap) fetch_h_.reserve(bytes + bytes / 2);
+    uint8_t* h = fetch_h_.ptr;
+    HostContacts r{};
+    auto copy = [&](const void* src, size_t b) {
+        uint8_t* at = h;
+        if (b) CC_CUDA(cudaMemcpyAsync(at, src, b, cudaMemcpyDeviceToHost, stream_));
+        h += b;
+        return at;
+    };
+    r.vertices = reinterpret_cast<const uint32_t*>(copy(c_verts_.ptr, 16 * n));
+    r.eps = reinterpret_cast<const double*>(copy(c_eps_.ptr, 8 * n));
+    r.radii = reinterpret_cast<const double*>(copy(radii_.ptr, 8 * m));
+    r.inc_off = reinterpret_cast<const uint64_t*>(h);
+    r.kinds = h + 8 * (m + 1);
+    r.counts = r.kinds + n;
+    copy(fetch_d_.ptr, dev);
+    // the counts may end off a 4-byte boundary
+    h = fetch_h_.ptr + ((size_t)(h - fetch_h_.ptr) + 3) / 4 * 4;
+    r.inc = reinterpret_cast<const uint32_t*>(copy(inc_, 4 * ni));
+    CC_CUDA(cudaStreamSynchronize(stream_));
+    return r;
 }
 
 }  // namespace cc

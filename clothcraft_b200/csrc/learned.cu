@@ -510,12 +510,12 @@ Mlp::Mlp(uint64_t seed) {
     fill(kOffW3, kMlpHidden, kMlpHidden, 1.0);
     fill(kOffW4, kMlpOut, kMlpHidden, 0.1);
     p_.upload(h, nullptr);
-    for (auto* b : {&m_, &v_, &g_}) {
+    for (auto* b : {&m_, &v_}) {
         b->reserve(kMlpParams);
         b->zero(kMlpParams, nullptr);
     }
-    loss_.reserve(1);
-    loss_.zero(1, nullptr);
+    g_.reserve(kMlpParams + 1);
+    g_.zero(kMlpParams + 1, nullptr);
     CC_CUDA(cudaStreamSynchronize(nullptr));
 }
 

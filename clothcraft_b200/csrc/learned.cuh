@@ -79,16 +79,20 @@ class Mlp {
     // Adam (Kingma & Ba 2015) with bias correction, one step.
     void adam(const float* grads, float lr, float beta1, float beta2, float eps, cudaStream_t st);
     float* grad_buffer() { return g_.ptr; }
-    float* loss_buffer() { return loss_.ptr; }
+    float* loss_buffer() { return g_.ptr + kMlpParams; }  // behind the gradient
     uint64_t adam_steps() const { return t_; }
 
-    // error word of the last tensor-core forward (1 = a bounded wait gave up)
-    unsigned int read_error(cudaStream_t st);
+    // whether a bounded wait of the last tensor-core forward gave up; waits for
+    // the stream. A wait gives up after kTcWaitNs, so a forward that was complete
+    // sooner than that cannot have failed and need not be asked about.
+    static constexpr uint64_t kTcWaitNs = 500ull * 1000 * 1000;
+    bool read_error(cudaStream_t st);
 
    private:
-    DBuf<float> p_, m_, v_, g_, loss_, partial_;
+    DBuf<float> p_, m_, v_, g_, partial_;  // g_: gradient and loss
     DBuf<__half> w16_;  // FP16 copies of W1..W4 in the tensor-core operand layout
-    DBuf<unsigned int> err_;
+    DBuf<unsigned int> err_;  // number of the last forward that failed: nothing to reset between forwards
+    unsigned int tc_forwards_ = 0;
     bool w16_valid_ = false;
     uint64_t t_ = 0;
     void refresh_half(cudaStream_t st);

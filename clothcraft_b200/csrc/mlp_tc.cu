@@ -12,6 +12,8 @@
 // frees the TMEM.
 #include <cuda_fp16.h>
 
+#include <atomic>
+
 #include "learned.cuh"
 
 namespace cc {
@@ -21,7 +23,7 @@ constexpr int kTcM = 128;       // samples per tile = TMEM lanes
 constexpr int kK1 = 32;         // layer-1 K (24 features padded)
 constexpr int kN4 = 16;         // output layer N (3 outputs padded; M = 128 needs N % 16 == 0)
 constexpr int kTmemCols = 128;  // [0,64) hidden accumulator, [64,80) output accumulator
-constexpr uint64_t kWaitNs = 500ull * 1000 * 1000;  // bound of every mbarrier wait (0.5 s)
+constexpr uint64_t kWaitNs = Mlp::kTcWaitNs;  // bound of every mbarrier wait (0.5 s)
 
 // Byte offset of element (row r, k) in a K-major, no-swizzle operand whose
 // rows hold `ktot` elements: 8x8 core matrices of 128 contiguous bytes,
@@ -48,9 +50,14 @@ constexpr uint32_t kSmH = kSmX + kXBytes;
 constexpr uint32_t kSmBar = kSmH + kHBytes;
 constexpr uint32_t kSmTmem = kSmBar + 8;
 constexpr uint32_t kSmBytes = kSmTmem + 8;
-// Dynamic shared memory requested per CTA: at least 57 KB so that no more
-// than 3 CTAs (384 TMEM columns of 512) share an SM.
-constexpr uint32_t kSmRequest = kSmBytes > 58 * 1024 ? kSmBytes : 58 * 1024;
+// Four CTAs share an SM, which their 128 TMEM columns each fill; shared memory
+// has no room for a fifth. A tile is a chain of short MMAs and long epilogues
+// (192 GELUs a thread), so what counts is how many tiles an SM has in flight: at
+// two CTAs per SM 65,536 samples took 36 us.
+constexpr int kTcBlocks = 4;
+constexpr uint32_t kSmRequest = kSmBytes;
+static_assert(kTcBlocks * kTmemCols <= 512, "TMEM columns of an SM");
+static_assert((kTcBlocks + 1) * (kSmRequest + 1024) > 228 * 1024, "no more CTAs per SM than the TMEM has columns for");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -164,10 +171,11 @@ __global__ void k_pack_half(const float* __restrict__ P, unsigned char* __restri
     }
 }
 
-__global__ void __launch_bounds__(128, 1) k_mlp_forward_tc(const float* __restrict__ P,
+__global__ void __launch_bounds__(128, kTcBlocks) k_mlp_forward_tc(const float* __restrict__ P,
                                                            const unsigned char* __restrict__ Wh,
                                                            const float* __restrict__ F, uint64_t n,
-                                                           float* __restrict__ out, unsigned int* err) {
+                                                           float* __restrict__ out, unsigned int* err,
+                                                                   unsigned int number) {
     extern __shared__ __align__(1024) unsigned char sm[];
     unsigned char* sW = sm + kSmW;
     unsigned char* sX = sm + kSmX;
@@ -283,7 +291,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_forward_tc(const float* __restri
         __syncthreads();
         fence_after();
     }
-    if (failed && tid == 0) atomicOr(err, 1u);
+    if (failed && tid == 0) atomicExch(err, number);
     fence_before();
     __syncthreads();
     fence_after();
@@ -302,22 +310,26 @@ void Mlp::refresh_half(cudaStream_t st) {
 
 void Mlp::forward_tc(const float* features, uint64_t n, float* out, cudaStream_t st) {
     refresh_half(st);
-    err_.reserve(1);
-    CC_CUDA(cudaMemsetAsync(err_.ptr, 0, sizeof(unsigned int), st));
-    allow_dynamic_smem(k_mlp_forward_tc, kSmRequest);
+    if (!err_.ptr) {
+        err_.reserve(1);
+        CC_CUDA(cudaMemsetAsync(err_.ptr, 0, sizeof(unsigned int), st));
+    }
+    if (++tc_forwards_ == 0u) tc_forwards_ = 1u;
+    static std::atomic<uint64_t> raised{0};  // devices on which the limit is raised
+    allow_dynamic_smem_once(k_mlp_forward_tc, kSmRequest, raised);
     uint64_t tiles = (n + kTcM - 1) / kTcM;
-    unsigned grid = (unsigned)std::min<uint64_t>(tiles, 148ull * 2ull);
+    unsigned grid = (unsigned)std::min<uint64_t>(tiles, 148ull * kTcBlocks);
     k_mlp_forward_tc<<<grid, 128, kSmRequest, st>>>(p_.ptr, reinterpret_cast<const unsigned char*>(w16_.ptr), features,
-                                                     n, out, err_.ptr);
+                                                     n, out, err_.ptr, tc_forwards_);
     CC_CUDA(cudaGetLastError());
 }
 
-unsigned int Mlp::read_error(cudaStream_t st) {
-    if (!err_.ptr) return 0;
+bool Mlp::read_error(cudaStream_t st) {
+    if (!err_.ptr) return false;
     unsigned int e = 0;
     CC_CUDA(cudaMemcpyAsync(&e, err_.ptr, sizeof e, cudaMemcpyDeviceToHost, st));
     CC_CUDA(cudaStreamSynchronize(st));
-    return e;
+    return e == tc_forwards_;
 }
 
 }  // namespace cc

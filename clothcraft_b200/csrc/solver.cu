@@ -416,6 +416,7 @@ struct cc_world {
     World* w = nullptr;
     cudaStream_t stream = nullptr;
     bool owns_stream = false;
+    Pinned<double4> stage;  // a call's positions on their way to the device
     std::string err;
     int code = 0;
     int fail(const Failure& f) {
@@ -434,6 +435,7 @@ struct cc_mlp {
     cudaStream_t stream = nullptr;
     DBuf<uint32_t> perm;
     DBuf<float> losses;
+    std::vector<float> grads_h;  // gradient and loss of a cc_mlp_gradients call
     std::string err;
     int code = 0;
     int fail(const Failure& f) {
@@ -1698,8 +1700,7 @@ int32_t cc_solver_colors(cc_solver* s, const double* x_all, double query_radius,
                          const cc_grab* grab, uint32_t* colors_out, uint32_t* n_colors) {
     try {
         if (!ogc_valid(*settings)) throw Failure{CC_ERR_INVALID_ARGUMENT, "Invalid OGC radius, stiffness or trust-region parameters"};
-        Pinned<double4> stage;
-        upload_all(s->world.get(), x_all, s->stream, stage);
+        upload_all(s->world.get(), x_all, s->stream, s->world_view.stage);
         s->world->detect(query_radius, settings->radius, settings->relaxation, settings->stiffness, true);
         s->coloring.compute(s->color_view(s->world->contacts(), grab), s->stream);
         std::vector<uint32_t> c;
@@ -1718,8 +1719,7 @@ int32_t cc_solver_local_blocks(cc_solver* s, const double* x_all, double query_r
     try {
         if (!ogc_valid(settings->contact))
             throw Failure{CC_ERR_INVALID_ARGUMENT, "Invalid OGC radius, stiffness or trust-region parameters"};
-        Pinned<double4> stage;
-        upload_all(s->world.get(), x_all, s->stream, stage);
+        upload_all(s->world.get(), x_all, s->stream, s->world_view.stage);
         size_t n = s->n;
         if (targets) {
             std::vector<double4> t(n);
@@ -1781,8 +1781,7 @@ int32_t cc_world_set_tree_rebuild_period(cc_world* w, int32_t period) {
 
 int32_t cc_world_validate_start(cc_world* w, const double* x) {
     try {
-        Pinned<double4> stage;
-        upload_all(w->w, x, w->w->stream(), stage);
+        upload_all(w->w, x, w->w->stream(), w->stage);
         w->w->validate_start();
         return CC_OK;
     } catch (const Failure& f) {
@@ -1797,17 +1796,12 @@ int32_t cc_world_detect(cc_world* w, const double* x, double query_radius, const
             throw Failure{CC_ERR_INVALID_ARGUMENT, "Invalid OGC radius, stiffness or trust-region parameters"};
         if (!std::isfinite(query_radius) || query_radius < settings->radius)
             throw Failure{CC_ERR_INVALID_ARGUMENT, "OGC query radius must cover the contact radius"};
-        Pinned<double4> stage;
-        upload_all(w->w, x, w->w->stream(), stage);
+        upload_all(w->w, x, w->w->stream(), w->stage);
         w->w->detect(query_radius, settings->radius, settings->relaxation, settings->stiffness, true);
         const DetectStats& st = w->w->stats();
-        std::vector<uint32_t> kind, verts, inc;
-        std::vector<double> eps, radii;
-        std::vector<uint64_t> inc_off;
-        w->w->download(kind, verts, eps, inc_off, inc, radii);
-        size_t moving = w->w->moving();
-        out->n_contacts = kind.size();
-        out->n_incident = inc.size();
+        const size_t n = st.n_contacts, n_inc = st.n_incident, moving = w->w->moving();
+        out->n_contacts = n;
+        out->n_incident = n_inc;
         out->active_contacts = st.active;
         out->vertex_face_candidates = st.vf_count;
         out->edge_edge_candidates = st.ee_count;
@@ -1815,18 +1809,19 @@ int32_t cc_world_detect(cc_world* w, const double* x, double query_radius, const
         out->aabb_rejections = st.rejections;
         std::memcpy(&out->minimum_distance, &st.min_dist_bits, 8);
         out->broad_phase_rebuilt = st.rebuild ? 1 : 0;
-        if (out->contact_capacity < kind.size() || out->incident_capacity < inc.size() || out->radii_capacity < moving)
+        if (out->contact_capacity < n || out->incident_capacity < n_inc || out->radii_capacity < moving)
             return CC_ERR_CAPACITY;
-        for (size_t c = 0; c < kind.size(); ++c) {
-            if (out->kinds) out->kinds[c] = (uint8_t)kind[c];
-            if (out->vertices)
-                for (int k = 0; k < 4; ++k) out->vertices[4 * c + k] = verts[4 * c + k];
-            if (out->counts) out->counts[c] = (uint8_t)(kind[c] == 0 ? 2 : (kind[c] == 1 ? 3 : 4));
-            if (out->mollifier_epsilon) out->mollifier_epsilon[c] = eps[c];
-        }
-        if (out->incident_offsets) std::copy(inc_off.begin(), inc_off.end(), out->incident_offsets);
-        if (out->incident) std::copy(inc.begin(), inc.end(), out->incident);
-        if (out->radii) std::copy(radii.begin(), radii.end(), out->radii);
+        const World::HostContacts c = w->w->fetch();
+        auto give = [](auto* to, const auto* from, size_t count) {
+            if (to && count) std::memcpy(to, from, count * sizeof(*from));
+        };
+        give(out->kinds, c.kinds, n);
+        give(out->vertices, c.vertices, 4 * n);
+        give(out->counts, c.counts, n);
+        give(out->mollifier_epsilon, c.eps, n);
+        give(out->incident_offsets, c.inc_off, moving + 1);
+        give(out->incident, c.inc, n_inc);
+        give(out->radii, c.radii, moving);
         return CC_OK;
     } catch (const Failure& f) {
         return w->fail(f);
@@ -1835,8 +1830,7 @@ int32_t cc_world_detect(cc_world* w, const double* x, double query_radius, const
 
 int32_t cc_world_candidates(cc_world* w, const double* x, double radius, cc_candidates* out) {
     try {
-        Pinned<double4> stage;
-        upload_all(w->w, x, w->w->stream(), stage);
+        upload_all(w->w, x, w->w->stream(), w->stage);
         std::vector<uint32_t> vf, ee;
         w->w->fresh_pairs(radius, vf, ee);
         out->n_vf = vf.size() / 2;
@@ -1920,9 +1914,11 @@ int32_t cc_mlp_forward(cc_mlp* m, const float* features, uint64_t n, float* out,
     try {
         if ((n && (!features || !out)) || (precision != 0 && precision != 1))
             throw Failure{CC_ERR_INVALID_ARGUMENT, "cc_mlp_forward: bad arguments"};
+        const double began = now_ms();
         m->net->forward(features, n, out, precision, m->stream);
         CC_CUDA(cudaStreamSynchronize(m->stream));
-        if (precision == 1 && m->net->read_error(m->stream))
+        // a call shorter than half the waits' bound cannot hold one that gave up
+        if (precision == 1 && (now_ms() - began) * 1e6 > 0.5 * (double)Mlp::kTcWaitNs && m->net->read_error(m->stream))
             throw Failure{CC_ERR_DEVICE_TIMEOUT, "tensor-core MLP: a bounded wait gave up"};
         return CC_OK;
     } catch (const Failure& f) {
@@ -1936,10 +1932,12 @@ int32_t cc_mlp_gradients(cc_mlp* m, const float* features, const float* targets,
         if (!features || !targets || !grads || !loss || n == 0)
             throw Failure{CC_ERR_INVALID_ARGUMENT, "cc_mlp_gradients: bad arguments"};
         m->net->gradients(features, targets, nullptr, n, m->net->grad_buffer(), m->net->loss_buffer(), m->stream);
-        CC_CUDA(cudaMemcpyAsync(grads, m->net->grad_buffer(), kMlpParams * sizeof(float), cudaMemcpyDeviceToHost,
-                                m->stream));
-        CC_CUDA(cudaMemcpyAsync(loss, m->net->loss_buffer(), sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+        m->grads_h.resize(kMlpParams + 1);
+        CC_CUDA(cudaMemcpyAsync(m->grads_h.data(), m->net->grad_buffer(), (kMlpParams + 1) * sizeof(float),
+                                cudaMemcpyDeviceToHost, m->stream));
         CC_CUDA(cudaStreamSynchronize(m->stream));
+        std::memcpy(grads, m->grads_h.data(), kMlpParams * sizeof(float));
+        *loss = m->grads_h[kMlpParams];
         return CC_OK;
     } catch (const Failure& f) {
         return m->fail(f);

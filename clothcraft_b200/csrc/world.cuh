@@ -161,9 +161,17 @@ class World {
     const TopologyHost& topology() const { return top_; }
     const uint32_t* nb_off() const { return nb_off_.ptr; }
     const uint32_t* nb() const { return nb_.ptr; }
-    // download the canonical contact set (for the C ABI / tests)
-    void download(std::vector<uint32_t>& kind, std::vector<uint32_t>& verts, std::vector<double>& eps,
-                  std::vector<uint64_t>& inc_off, std::vector<uint32_t>& inc, std::vector<double>& radii);
+    // The canonical contact set of the last detection in host memory, in the
+    // types of cc_contacts; the pointers hold until the next call.
+    struct HostContacts {
+        const uint32_t* vertices;  // [n_contacts][4]
+        const double* eps;
+        const double* radii;       // [moving]
+        const uint64_t* inc_off;   // [moving + 1]
+        const uint32_t* inc;
+        const uint8_t *kinds, *counts;
+    };
+    HostContacts fetch();
     cudaStream_t stream() const { return stream_; }
     void invalidate_cache() { cache_valid_ = false; }
     uint64_t launches() const { return launches_; }
@@ -243,6 +251,8 @@ class World {
     double* inc_eps_ = nullptr;
     uint32_t *inc_ = nullptr, *inc_raw_ = nullptr;
     RadixSorter sorter_;
+    DBuf<uint8_t> fetch_d_;    // kinds, counts and 64-bit offsets of fetch()
+    Pinned<uint8_t> fetch_h_;
     DBuf<uint32_t> scan_tmp_;
     DBuf<DetectStats> stats_d_;
     Pinned<DetectStats> stats_h_;
