@@ -166,6 +166,15 @@ inline void allow_dynamic_smem_once(K* kernel, size_t bytes, std::atomic<uint64_
     if (bit) raised.fetch_or(bit, std::memory_order_acq_rel);
 }
 
+// Programmatic dependent launch: a launch may start while the launch before it
+// drains. wait_for_last_launch returns once that launch is complete and its
+// writes are visible; only then does the block let the next launch start, so
+// whatever runs before the wait can rely on every launch but the last.
+__device__ __forceinline__ void wait_for_last_launch() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Launches a kernel that may start while the launch before it in the stream
 // drains (programmatic dependent launch); the kernel waits for that launch
 // itself (griddepcontrol.wait) before it reads what it wrote.

@@ -156,6 +156,7 @@ constexpr int kResidualLanes = 4;
 // iterate of the next call).
 __global__ void k_accelerate(uint32_t n, const uint8_t* pinned, ContactsView c, double4* x, double4* hist,
                              const StepScalars* sc, uint32_t it) {
+    wait_for_last_launch();
     if (sc->stop_at <= it) return;  // this iteration was skipped
     const bool extrapolate = sc->acc_k >= 2;
     const double w = sc->acc_w;
@@ -240,6 +241,7 @@ __global__ void k_warm_start(uint32_t n, const uint8_t* pinned, const double4* g
 // projective and position-based dynamics"): w1 = 1, w2 = 2/(2 - rho^2),
 // wk = 4/(4 - rho^2 w(k-1)), rounded operation by operation as on the CPU.
 __global__ void k_refresh_rule(StepScalars* sc, uint32_t it, uint32_t iterations, double threshold, double rho2) {
+    wait_for_last_launch();
     if (sc->stop_at <= it) return;  // this iteration was skipped
     if (rho2 > 0.0) {
         unsigned int k = ++sc->acc_k;
@@ -267,6 +269,7 @@ __global__ void k_refresh_rule(StepScalars* sc, uint32_t it, uint32_t iterations
 __global__ void __launch_bounds__(256) k_residual_rule(StepScalars* sc, const double* partial, uint32_t it,
                                                        uint32_t iterations, double tol2, int stop, uint32_t stall,
                                                        int accelerate) {
+    wait_for_last_launch();
     if (sc->stop_at <= it) return;  // uniform: every thread reads it before thread 0 writes
     double g2 = block_sum_partials(partial);
     if (threadIdx.x == 0) {
@@ -1037,9 +1040,9 @@ void cc_solver::step(const cc_vbd_settings& s, const cc_grab* grab, cc_metrics* 
                     sweep(sv, coloring.order() + off[c], cnt, fp32);
                     ++own_launches;
                 }
-                k_refresh_rule<<<1, 1, 0, stream>>>(sc.ptr, it, s.iterations, threshold, rho2);
+                launch_after(k_refresh_rule, 1, 1, stream, sc.ptr, it, s.iterations, threshold, rho2);
                 if (accelerate) {
-                    k_accelerate<<<gb, 256, 0, stream>>>(n, pinned.ptr, cv, world->x(), acc_prev2, sc.ptr, it);
+                    launch_after(k_accelerate, gb, 256, stream, n, pinned.ptr, cv, world->x(), acc_prev2, sc.ptr, it);
                     std::swap(acc_prev1, acc_prev2);
                     ++own_launches;
                 }
@@ -1047,8 +1050,8 @@ void cc_solver::step(const cc_vbd_settings& s, const cc_grab* grab, cc_metrics* 
                 if (checks && ((it + 1) % check_every == 0 || it + 1 == s.iterations)) {
                     launch_grad_sq(sv, gsq.ptr, &sc.ptr->stop_at, it, kResidualLanes, true, stream);
                     launch_sum_partial(gsq.ptr, n, partial.ptr, &sc.ptr->stop_at, it, stream);
-                    k_residual_rule<<<1, 256, 0, stream>>>(sc.ptr, partial.ptr, it, s.iterations, tol2,
-                                                           target_on ? 1 : 0, s.stall_refresh, accelerate ? 1 : 0);
+                    launch_after(k_residual_rule, 1, 256, stream, sc.ptr, partial.ptr, it, s.iterations, tol2,
+                                 target_on ? 1 : 0, s.stall_refresh, accelerate ? 1 : 0);
                     own_launches += 3;
                 }
             }

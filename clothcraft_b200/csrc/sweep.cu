@@ -23,15 +23,6 @@
 
 namespace cc {
 
-// Programmatic dependent launch: a sweep launch may start while the launch
-// before it drains. wait_for_last_launch returns once that launch is complete
-// and its writes are visible; only then does the block let the next launch
-// start, so whatever runs before the wait can rely on every launch but the last.
-__device__ __forceinline__ void wait_for_last_launch() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // Solves vertex i of the colour; `wait`: the group's first vertex of the launch.
 // False if the launch is to be skipped.
 template <int G>
@@ -359,13 +350,19 @@ template <int G>
 __global__ void __launch_bounds__(128) k_grad_sq(SweepView s, double* out, const unsigned* skip_at, uint32_t iteration,
                                                  int project) {
     __shared__ double near_s[128 / G * Near<G>::kDoubles];
-    if (skip_at && *skip_at <= iteration) return;
     uint32_t t = blockIdx.x * 128 + threadIdx.x;
     uint32_t v = t / G;
     if (v >= s.n) return;  // whole groups leave together
     uint32_t lane = threadIdx.x & (G - 1);
     unsigned mask = G >= 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1)));
-    if (s.pinned[v]) {
+    Near<G> T;
+    T.head(s, v);
+    const bool pinned = s.pinned[v] != 0;
+    const typename Near<G>::Ids ids = T.ids(s, lane);
+    const typename Near<G>::First f = T.first(s, lane);
+    wait_for_last_launch();
+    if (skip_at && *skip_at <= iteration) return;
+    if (pinned) {
         if (lane == 0) out[v] = 0.0;
         return;
     }
@@ -373,9 +370,7 @@ __global__ void __launch_bounds__(128) k_grad_sq(SweepView s, double* out, const
     d3 g = mk(0, 0, 0);
     Sym H;
     sym_zero(H);
-    Near<G> T;
-    T.head(s, v);
-    const typename Near<G>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
+    T.stage(s, ids, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
     local_part<true, G, false>(s, T, f, x, lane, g, H);  // gradient only
     if (G > 1) {
         g.x = group_sum<G>(g.x, mask);
@@ -399,12 +394,12 @@ void launch_grad_sq(const SweepView& s, double* out, const unsigned* skip_at, ui
     if (grid == 0) return;
     int p = project ? 1 : 0;
     switch (G) {
-        case 1: k_grad_sq<1><<<grid, 128, 0, st>>>(s, out, skip_at, iteration, p); break;
-        case 2: k_grad_sq<2><<<grid, 128, 0, st>>>(s, out, skip_at, iteration, p); break;
-        case 4: k_grad_sq<4><<<grid, 128, 0, st>>>(s, out, skip_at, iteration, p); break;
-        case 16: k_grad_sq<16><<<grid, 128, 0, st>>>(s, out, skip_at, iteration, p); break;
-        case 32: k_grad_sq<32><<<grid, 128, 0, st>>>(s, out, skip_at, iteration, p); break;
-        default: k_grad_sq<8><<<grid, 128, 0, st>>>(s, out, skip_at, iteration, p); break;
+        case 1: launch_after(k_grad_sq<1>, grid, 128, st, s, out, skip_at, iteration, p); break;
+        case 2: launch_after(k_grad_sq<2>, grid, 128, st, s, out, skip_at, iteration, p); break;
+        case 4: launch_after(k_grad_sq<4>, grid, 128, st, s, out, skip_at, iteration, p); break;
+        case 16: launch_after(k_grad_sq<16>, grid, 128, st, s, out, skip_at, iteration, p); break;
+        case 32: launch_after(k_grad_sq<32>, grid, 128, st, s, out, skip_at, iteration, p); break;
+        default: launch_after(k_grad_sq<8>, grid, 128, st, s, out, skip_at, iteration, p); break;
     }
 }
 
@@ -449,6 +444,7 @@ void launch_term_energy(const SweepView& s, const ObjectiveCounts& c, double* ou
 // Deterministic sum, first pass: kSumBlocks fixed-order partial sums.
 __global__ void __launch_bounds__(256) k_sum_partial(const double* v, uint64_t n, double* partial,
                                                      const unsigned* skip_at, uint32_t iteration) {
+    wait_for_last_launch();
     if (skip_at && *skip_at <= iteration) return;
     __shared__ double sh[256];
     double a = 0.0;
@@ -464,7 +460,7 @@ __global__ void __launch_bounds__(256) k_sum_partial(const double* v, uint64_t n
 
 void launch_sum_partial(const double* v, uint64_t n, double* partial, const unsigned* skip_at, uint32_t iteration,
                         cudaStream_t st) {
-    k_sum_partial<<<kSumBlocks, 256, 0, st>>>(v, n, partial, skip_at, iteration);
+    launch_after(k_sum_partial, kSumBlocks, 256, st, v, n, partial, skip_at, iteration);
 }
 
 
