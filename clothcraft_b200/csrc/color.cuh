@@ -10,6 +10,8 @@ struct ColorView {
     uint32_t n;
     const uint32_t* lo_off;  // [n+1] lower-index neighbours of the material graph
     const uint32_t* lo;
+    const uint4* head;       // [2n] .x, .y of each pair: first entry and length of the vertex's list in nb
+    const uint32_t* nb;      // neighbours of the material graph
     ContactsView contacts;
     uint64_t n_incident;  // entries of contacts.inc
     int grab_active;
@@ -33,19 +35,20 @@ class Coloring {
     uint64_t launches() const { return launches_; }
 
    private:
-    static constexpr int kBatch = 8;
     uint32_t n_ = 0;
     uint64_t lo_total_ = 0;
     DBuf<uint32_t> adj_;   // distinct lower neighbours of every vertex (k_color_rows)
     DBuf<uint4> row_head_;
     DBuf<uint16_t> a_, b_;
     uint16_t* cur_ = nullptr;
-    DBuf<uint32_t> order_, counts_, iota_;
+    DBuf<uint32_t> order_, iota_;
+    // a colouring's words, cleared and read back as one: rounds, error, n - first failing vertex, (unused), vertices
+    // per colour; behind them (not read back) the walk's dirty bits
+    static constexpr size_t kWords = 4 + kMaxColors;
+    DBuf<uint32_t> words_;
+    Pinned<uint32_t> words_h_;
     RadixSorter sorter_;
     unsigned int* error_word_ = nullptr;  // receives DERR_SORT_WAIT (set_error_word)
-    DBuf<unsigned int> changed_;
-    Pinned<unsigned int> changed_h_;
-    Pinned<uint32_t> counts_h_;
     std::vector<uint32_t> offsets_h_;
     uint32_t n_colors_ = 0;
     size_t last_iterations_ = 0;

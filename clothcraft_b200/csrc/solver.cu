@@ -595,6 +595,8 @@ struct cc_solver {
         c.n = n;
         c.lo_off = lo_off.ptr;
         c.lo = lo.ptr;
+        c.head = vt.head;
+        c.nb = vt.nb;
         c.contacts = cv;
         c.n_incident = world->stats().n_incident;
         c.grab_active = grab ? 1 : 0;
