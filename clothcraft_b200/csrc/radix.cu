@@ -1,5 +1,6 @@
 // Stable LSD radix sort and prefix sums (see radix.cuh).
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "radix.cuh"
@@ -198,6 +199,88 @@ __global__ void __launch_bounds__(kBlock) k_onesweep_pass(const K* __restrict__ 
     }
 }
 
+// Up to kSmallMax keys: every pass in one block, keys and their places in shared
+// memory. The multi-launch form takes two launches and one a pass (11 for a
+// 64-bit key, ~3 us each in a stream) whatever the size; this takes one launch of
+// ~2 us a pass at 1,024 keys, ~3.5 at 2,048.
+constexpr int kSmallBlock = 1024;
+constexpr int kSmallItems = 2;
+constexpr int kSmallMax = kSmallBlock * kSmallItems;
+constexpr int kSmallGroups = kSmallMax / 32;  // 32 consecutive keys each, counted by one warp
+template <class K>
+constexpr size_t small_bytes() {
+    return kSmallMax * 2 * sizeof(K) + kSmallMax * 2 * sizeof(uint16_t) + kSmallGroups * kRadix * sizeof(uint16_t) +
+           5 * kRadix * sizeof(uint32_t);
+}
+
+template <class K, class V>
+__global__ void __launch_bounds__(kSmallBlock) k_sort_small(const K* __restrict__ kin, K* __restrict__ kout,
+                                                            const V* __restrict__ vin, V* __restrict__ vout, uint32_t n,
+                                                            int bits) {
+    extern __shared__ __align__(16) unsigned char small_sm[];
+    K* key = reinterpret_cast<K*>(small_sm);                                     // [2][kSmallMax]
+    uint32_t* part = reinterpret_cast<uint32_t*>(key + 2 * kSmallMax);           // [4][kRadix] counts by quarter
+    uint32_t* start = part + 4 * kRadix;                                         // [kRadix] keys of lower digits
+    uint16_t* place = reinterpret_cast<uint16_t*>(start + kRadix);               // [2][kSmallMax] input places
+    uint16_t* cnt = place + 2 * kSmallMax;                                       // [kSmallGroups][kRadix]
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, d = t & (kRadix - 1), q = t / kRadix;
+    for (uint32_t i = t; i < n; i += kSmallBlock) {
+        key[i] = kin[i];
+        place[i] = (uint16_t)i;
+    }
+    int cur = 0;
+    for (int shift = 0; shift < bits; shift += 8) {
+        const int width = bits - shift < 8 ? bits - shift : 8;
+        const uint32_t mask = (1u << width) - 1u;
+        for (uint32_t i = t; i < kSmallGroups * kRadix / 8; i += kSmallBlock)
+            reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+        const K* src = key + cur * kSmallMax;
+        uint32_t dig[kSmallItems], rank[kSmallItems];
+#pragma unroll
+        for (int j = 0; j < kSmallItems; ++j) {
+            const uint32_t i = j * kSmallBlock + t;
+            dig[j] = i < n ? (uint32_t)(src[i] >> shift) & mask : (uint32_t)kRadix;
+            const unsigned peers = __match_any_sync(0xffffffffu, dig[j]);
+            rank[j] = __popc(peers & ((1u << lane) - 1u));
+            if (i < n && rank[j] == 0) cnt[(j * (kSmallBlock / 32) + warp) * kRadix + dig[j]] = (uint16_t)__popc(peers);
+        }
+        __syncthreads();
+        // keys of digit d in the groups of quarter q, and before each group
+        constexpr uint32_t kQuarter = kSmallGroups / 4;
+        uint32_t sum = 0;
+        for (uint32_t g = q * kQuarter; g < (q + 1) * kQuarter; ++g) {
+            const uint32_t c = cnt[g * kRadix + d];
+            cnt[g * kRadix + d] = (uint16_t)sum;
+            sum += c;
+        }
+        part[q * kRadix + d] = sum;
+        __syncthreads();
+        const uint32_t all = t < kRadix ? part[d] + part[kRadix + d] + part[2 * kRadix + d] + part[3 * kRadix + d] : 0u;
+        uint32_t total;
+        const uint32_t before = block_exclusive_scan<uint32_t, kSmallBlock>(all, total);
+        if (t < kRadix) start[d] = before;
+        __syncthreads();
+        K* dst = key + (cur ^ 1) * kSmallMax;
+#pragma unroll
+        for (int j = 0; j < kSmallItems; ++j) {
+            const uint32_t i = j * kSmallBlock + t;
+            if (i >= n) continue;
+            const uint32_t g = j * (kSmallBlock / 32) + warp;
+            uint32_t pos = start[dig[j]] + cnt[g * kRadix + dig[j]] + rank[j];
+            for (uint32_t k = 0; k < g / kQuarter; ++k) pos += part[k * kRadix + dig[j]];
+            dst[pos] = src[i];
+            place[(cur ^ 1) * kSmallMax + pos] = place[cur * kSmallMax + i];
+        }
+        cur ^= 1;
+        __syncthreads();
+    }
+    for (uint32_t i = t; i < n; i += kSmallBlock) {
+        kout[i] = key[cur * kSmallMax + i];
+        if constexpr (!std::is_same<V, NoValue>::value) vout[i] = vin[place[cur * kSmallMax + i]];
+    }
+}
+
 // ------------------------------------------------------------ prefix sums
 template <class T>
 __global__ void __launch_bounds__(kBlock) k_tile_reduce(const T* __restrict__ in, size_t n, T* __restrict__ partial) {
@@ -263,6 +346,14 @@ int RadixSorter::sort_impl(const K* keys_in, K* keys_out, const V* vals_in, V* v
     }
     if (n > kCountMask) throw Failure{CC_ERR_INVALID_ARGUMENT, "radix sort: more than 2^30 keys"};
     if (bits > 8 * kMaxPasses) throw Failure{CC_ERR_INVALID_ARGUMENT, "radix sort: more than 64 key bits"};
+    if (n <= kSmallMax) {
+        constexpr size_t smem = small_bytes<K>();
+        static std::atomic<uint64_t> raised{0};  // devices on which the limit is raised
+        allow_dynamic_smem_once(k_sort_small<K, V>, smem, raised);
+        k_sort_small<K, V><<<1, kSmallBlock, smem, s>>>(keys_in, keys_out, vals_in, vals_out, (uint32_t)n, bits);
+        CC_CUDA(cudaGetLastError());
+        return 1;
+    }
     const int passes = (bits + 7) / 8;
     const uint32_t tiles = (uint32_t)((n + kTile - 1) / kTile);
     // per pass: kRadix digit offsets, a tile counter, tiles x kRadix status words

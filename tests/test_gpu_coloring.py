@@ -60,3 +60,18 @@ def test_walk_equals_sequential_greedy(nx, ny, count, gap, rq, permute, least):
         co, no = o.colors(x, rq, sc.settings.ogc_c(), grab=gr)
         assert ng == no and ng >= least
         assert np.array_equal(cg, co)
+
+
+@pytest.mark.parametrize("nx,ny", [(2, 2), (33, 32), (33, 33), (2, 1026), (41, 50), (32, 64), (3, 683)])
+def test_small_sorts_around_their_limit(nx, ny):
+    """Triangle counts 2, 1984, 2048 and 2050 (the extension metric's sort), vertex counts 2050, 2048 and 2049 (the
+    colour order): a step takes every vertex in its colour's turn and reports the metric of the sorted strains."""
+    sc = layers(nx, ny, 1, 1e-3, "random", seed=nx)
+    st = sc.settings.to_c()
+    x, v, t, m = VbdSolver(sc).step(sc.x0, sc.v0, 0.0, st)
+    xo, vo, to, mo = oracle.Solver(sc, threads=8).step(sc.x0, sc.v0, 0.0, st)
+    # positions as in the other one-step comparisons; the metric moves with them by 100 / (4 mm spacing) per metre
+    assert np.abs(x - xo).max() <= 1e-9
+    assert abs(m["extension_p95_percent"] - mo["extension_p95_percent"]) <= 1e-4
+    assert abs(m["extension_max_percent"] - mo["extension_max_percent"]) <= 1e-4
+    assert m["extension_max_percent"] >= m["extension_p95_percent"] > 0.0
