@@ -8,7 +8,7 @@
 // the unique solution of  c(v) = mex { c(u) : u ~ v, u < v }.  A plain
 // parallel fixed-point iteration of that system needs as many sweeps as the
 // longest descending chain, and contact edges between folded layers make
-// chains of length ~n; k_color_chunked below bounds the work by walking
+// chains of length ~n; k_color_walk below bounds the work by walking
 // index-ordered chunks instead.
 
 #include <algorithm>

@@ -177,7 +177,9 @@ __device__ __forceinline__ void wait_for_last_launch() {
 
 // Launches a kernel that may start while the launch before it in the stream
 // drains (programmatic dependent launch); the kernel waits for that launch
-// itself (griddepcontrol.wait) before it reads what it wrote.
+// itself (wait_for_last_launch) before it reads what it wrote. A chain of short
+// launches is bound by each one's start and first loads: the sweeps of a 16-vertex
+// patch went 0.630 -> 0.563 ms a step (96 launches), of the fold 7.27 -> 7.08.
 template <class... P, class... A>
 inline void launch_after(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A&&... args) {
     cudaLaunchConfig_t c{};

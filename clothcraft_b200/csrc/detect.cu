@@ -618,7 +618,12 @@ __device__ __forceinline__ unsigned long long append_slot(unsigned long long* co
 // Pairs of one query, gathered in the thread's column of shared memory and
 // appended to the list 16 at a time: one atomic with its round trip per 16 pairs
 // instead of one per accepted leaf, and runs of one query in the list, whose
-// gathers the narrow phase's neighbouring lanes share.
+// gathers the narrow phase's neighbouring lanes share. The queries are bound by
+// the latency of their walks; with the leaf records (no lookups per accepted leaf)
+// a rebuild with its tree refits went 0.65 -> 0.42 ms on a 40k-vertex garment and
+// 1.0 -> 0.67 on the fold, and the narrow phase gained 12 to 17 %. Records of four
+// grandchildren (two levels a visit) were slower: the garment's detections of a
+// step 15.6 -> 17.1 ms.
 constexpr int kQueryBlock = 128;
 constexpr uint32_t kPairBuffer = 16;
 struct PairSink {
@@ -775,7 +780,8 @@ __device__ __forceinline__ void push_ee(const NarrowOut& o, uint32_t e, uint2 id
 // instead of on the ~quarter of the lanes whose pair is in range. Boxes are formed
 // from the positions, which a pair that is not rejected needs anyway (min and max
 // are exact: the same boxes as k_refit's), one dependent load less than
-// reading them. Bound by those gathers (pair -> vertices -> positions).
+// reading them. Bound by those gathers (pair -> vertices -> positions). With its
+// canonical set, a detection of a 640 x 640 crumple (38 M pairs) 2.5 -> 2.0 ms.
 constexpr int kNarrowBlock = 128;
 constexpr uint32_t kNarrowQueue = 64;
 enum NarrowTest : uint32_t { TEST_VERTEX = 0, TEST_EDGE = 1, TEST_EDGES = 2 };

@@ -250,7 +250,8 @@ __global__ void __launch_bounds__(kFwdBlock) k_mlp_forward_f32(const float* __re
 // are for the backward one, activations unit-major (a row of kPitch samples), so
 // that both sides of every product are contiguous float4. One thread per sample
 // and unit range, weights from global memory and one weight gradient per thread
-// at two shared-memory reads per FMA, took 290 us for the 16,384.
+// at two shared-memory reads per FMA, took 315 us for the 16,384; this takes 58
+// (clocks and caches as a launch-by-launch profile leaves them).
 constexpr int kTile = 64;
 constexpr int kPitch = kTile + 4;  // float4 rows; rows r and r + 1 lie 4 banks apart
 constexpr int kTrainBlock = 256;

@@ -10,7 +10,8 @@
 // (decoupled look-back), then scatters. A block only ever waits on blocks
 // that started before it, and each wait is bounded: a look-back that gives
 // up sets an error bit in the caller's error word instead of hanging.
-// Stability keeps equal keys in input order, so the passes order by the whole
+// Up to 2,048 keys one block does every pass in shared memory instead (one
+// launch; k_sort_small). Stability keeps equal keys in input order, so the passes order by the whole
 // key; the inputs are left untouched.
 #pragma once
 #include "common.cuh"

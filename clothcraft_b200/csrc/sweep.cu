@@ -16,9 +16,20 @@
 // line-search decisions without a broadcast.
 //
 // This is the FP64 form (cc_vbd_settings.sweep_precision = CC_SWEEP_FP64):
-// every term and the 3x3 solve in FP64, operation for operation as the CPU
-// path, so that GPU and CPU iterates agree to the last bits. sweep32.cu holds
-// the FP32-assembly form.
+// every term and the 3x3 solve in FP64, with derivatives in closed form where
+// the CPU path differentiates forward, so that GPU and CPU iterates agree to
+// rounding (~1e-16 m a step). sweep32.cu holds the FP32-assembly form.
+//
+// What bounds it: the latency of a solve's chain (head -> ids and records ->
+// positions -> ~2,000 warp instructions of mostly dependent FP64 arithmetic, twice
+// with the line search) at the 12 to 16 warps that its registers leave an SM; on
+// the fold the FP64 pipe is 27 % busy, issue 35 %, DRAM 12 %. Hence the order of the loads
+// (solve_vertex), the records (VertexTerms), the positions staged once (Near) and
+// the launches that start while the last one drains (launch_after). A launch on
+// the fold (16k vertices, 8 lanes, cold caches): 39.9 us with per-element data and
+// generic second derivatives (spilling at 128 registers), 26.6 us now (168, none); a 640 x 640 crumple's sweeps of a step
+// (410k vertices, 40 iterations) 31.1 -> 21.5 ms. With the records in their loops
+// instead of loaded ahead, the crumple took 27.2 ms.
 #include "sweep_terms.cuh"
 
 namespace cc {

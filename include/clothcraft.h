@@ -103,8 +103,8 @@ enum cc_init_mode {
 };
 /* Arithmetic of the colour sweeps (no reference counterpart; the reference's
  * CPU path is FP64, its wgpu shader FP32).
- * CC_SWEEP_FP64: every term and the 3x3 solve in FP64, operation for operation
- *   as the CPU path (the parity form).
+ * CC_SWEEP_FP64: every term and the 3x3 solve in FP64 (the parity form: it
+ *   agrees with the CPU path to rounding).
  * CC_SWEEP_FP32: membrane and bending energies, gradients and Hessians in FP32
  *   from FP64 edge differences; OGC contact terms in FP64; the 3x3 solve in
  *   FP32 unless its condition estimate exceeds 1e6; the line search compares
@@ -292,9 +292,10 @@ uint64_t cc_solver_total(const cc_solver* solver);
  * src/gpu_vbd/cache.rs:16-33). */
 void* cc_solver_stream(const cc_solver* solver);
 /* When enabled, each chunk of iterations the step enqueues ahead of the
- * device (all iterations without a residual target; max(check_every, 4)
- * with one) is captured into a CUDA graph and launched as one, except the
- * first iteration after each detection, which is launched directly so that
+ * device (without a residual target one iteration, four more, then eight at a
+ * time and the rest in powers of two; max(check_every, 4) with one) is
+ * captured into a CUDA graph and launched as one, except the first
+ * iteration after each detection, which is launched directly so that
  * the device works while the rest of its chunk is captured. Executable
  * graphs are kept per chunk shape (colour count, placement of the residual
  * checks) and updated in place while the shape recurs.
