@@ -1405,8 +1405,8 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
             mid[v] = make_uint2(hb, sb);
             head[2 * v] = make_uint4((uint32_t)nb.size(), (uint32_t)graph[v].size(), n_vt_tri, hb - io[v]);
             head[2 * v + 1] = make_uint4(n_vt_hinge, ends, sb - hb - ends, io[v + 1] - sb);
-            if (graph[v].size() >> 21)  // the records' 21-bit places
-                throw Failure{CC_ERR_INVALID_ARGUMENT, "a vertex has more than 2^21 mesh neighbours"};
+            if (graph[v].size() > kSelfPlace)  // the records' 21-bit places
+                throw Failure{CC_ERR_INVALID_ARGUMENT, "a vertex has 2^21 mesh neighbours or more"};
             nb.insert(nb.end(), graph[v].begin(), graph[v].end());
             n_vt_tri += hb - io[v];
             n_vt_hinge += sb - hb;

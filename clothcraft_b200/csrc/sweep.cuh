@@ -27,7 +27,8 @@ struct GrabDev {
 
 // A vertex's elastic terms as the local solves read them (k_vertex_terms): one
 // record per (vertex, term), a vertex's records side by side, with the term's
-// other vertices named by their place in the vertex's neighbour list and the
+// other vertices named by their place in the vertex's neighbour list (kSelfPlace:
+// the vertex itself) and the
 // element data turned to the vertex's point of view. A solve then reads one head,
 // one list of ids and one position per neighbour, and coalesced records, where
 // per-element data took head -> entry -> element -> positions, with each
@@ -43,6 +44,10 @@ struct VertexTerms {
 };
 
 constexpr uint32_t kPinnedHead = ~0u;
+// The place of the vertex itself, which its neighbour list leaves out: a hinge can
+// name a vertex twice (two faces on the same three vertices have one vertex as both
+// wings).
+constexpr uint32_t kSelfPlace = (1u << 21) - 1u;
 
 struct SweepView {
     uint32_t n;                 // moving vertices
