@@ -77,10 +77,10 @@ def load_peaks():
 # launch on the fold, from one ncu capture of the profiling driver (the first
 # sweep launch of a 30-iteration step from the fold-phase state; cold cache,
 # since ncu flushes the caches between its passes):
-#   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:k_sweep -s 0 -c 2 \
+#   ncu --set full --clock-control none -k regex:k_sweep -s 0 -c 2 \
 #       python -m clothcraft_b200.profile_fold --steps 1 --lanes 776 --fixed 30
-# (first launch: 25,242,624 B read, none written)
-SWEEP_TRAFFIC_BYTES = 25242624.0
+# (first launch: 25,243,136 B read, none written)
+SWEEP_TRAFFIC_BYTES = 25243136.0
 
 
 def workload():
