@@ -96,6 +96,8 @@ struct Pinned {
     void reserve(size_t n) {
         if (n <= cap) return;
         if (ptr) cudaFreeHost(ptr);
+        ptr = nullptr;  // empty if the allocation fails
+        cap = 0;
         CC_CUDA(cudaMallocHost(&ptr, (n ? n : 1) * sizeof(T)));
         cap = n;
     }
