@@ -1357,6 +1357,7 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
         uint64_t Hn = mesh->n_hinges;
         std::vector<uint4> hv(Hn);
         std::vector<double> hk(Hn);
+        std::vector<uint8_t> twice(n, 0);  // vertices that a hinge names twice: their records name the vertex itself
         for (uint64_t i = 0; i < Hn; ++i) {
             const uint32_t* v = mesh->hinges + 4 * i;
             for (int k = 0; k < 4; ++k)
@@ -1371,6 +1372,9 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
             hv[i] = make_uint4(v[0], v[1], v[2], v[3]);
             hk[i] = 0.5 * mesh->hinge_weight[i] * (M.bend_warp * aw * aw + M.bend_weft * af * af);
             for (uint32_t k = 0; k < 4; ++k) inc[v[k]].push_back(pack_term(TERM_HINGE, k, (uint32_t)i));
+            for (uint32_t k = 1; k < 4; ++k)
+                for (uint32_t j = 0; j < k; ++j)
+                    if (v[j] == v[k]) twice[v[k]] = 1;
             connect(v, 4);
         }
         h->n_stitch = (uint32_t)S;
@@ -1403,11 +1407,13 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
                 else if (type == TERM_HINGE) ++sb, ends += ((e >> 28) & 3u) < 2u ? 1u : 0u;
             }
             mid[v] = make_uint2(hb, sb);
-            head[2 * v] = make_uint4((uint32_t)nb.size(), (uint32_t)graph[v].size(), n_vt_tri, hb - io[v]);
-            head[2 * v + 1] = make_uint4(n_vt_hinge, ends, sb - hb - ends, io[v + 1] - sb);
-            if (graph[v].size() > kSelfPlace)  // the records' 21-bit places
-                throw Failure{CC_ERR_INVALID_ARGUMENT, "a vertex has 2^21 mesh neighbours or more"};
+            const size_t nb0 = nb.size();
             nb.insert(nb.end(), graph[v].begin(), graph[v].end());
+            if (twice[v]) nb.insert(std::lower_bound(nb.begin() + nb0, nb.end(), (uint32_t)v), (uint32_t)v);
+            if ((nb.size() - nb0) >> 21)  // the records' 21-bit places
+                throw Failure{CC_ERR_INVALID_ARGUMENT, "a vertex has more than 2^21 mesh neighbours"};
+            head[2 * v] = make_uint4((uint32_t)nb0, (uint32_t)(nb.size() - nb0), n_vt_tri, hb - io[v]);
+            head[2 * v + 1] = make_uint4(n_vt_hinge, ends, sb - hb - ends, io[v + 1] - sb);
             n_vt_tri += hb - io[v];
             n_vt_hinge += sb - hb;
             iv.insert(iv.end(), inc[v].begin(), inc[v].end());

@@ -308,7 +308,6 @@ __global__ void k_vertex_terms(SweepView s, unsigned long long* tri, double4* tr
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < s.n; v += gridDim.x * blockDim.x) {
         const uint4 a = s.vt.head[2 * (size_t)v], b = s.vt.head[2 * (size_t)v + 1];
         auto place = [&](uint32_t id) {  // in the ascending neighbour list
-            if (id == v) return (unsigned long long)kSelfPlace;
             uint32_t lo = 0, hi = a.y;
             while (lo < hi) {
                 const uint32_t mid = (lo + hi) >> 1;

@@ -27,8 +27,7 @@ struct GrabDev {
 
 // A vertex's elastic terms as the local solves read them (k_vertex_terms): one
 // record per (vertex, term), a vertex's records side by side, with the term's
-// other vertices named by their place in the vertex's neighbour list (kSelfPlace:
-// the vertex itself) and the
+// other vertices named by their place in the vertex's neighbour list and the
 // element data turned to the vertex's point of view. A solve then reads one head,
 // one list of ids and one position per neighbour, and coalesced records, where
 // per-element data took head -> entry -> element -> positions, with each
@@ -36,7 +35,9 @@ struct GrabDev {
 struct VertexTerms {
     const uint4* head;  // [2n] {first neighbour, neighbours, first triangle record, triangles},
                         //      {first hinge record, edge-end hinges, wing hinges, stitches}
-    const uint32_t* nb;                // neighbour ids, ascending (the material graph)
+    // neighbour ids, ascending (the material graph); a vertex that a hinge names twice (two faces on the same three
+    // vertices have one vertex as both wings) is in its own list
+    const uint32_t* nb;
     const unsigned long long* tri;     // neighbours j | k << 21 | material << 42
     const double4* tri_b;              // fibre vectors w = dj b.x + dk b.y, v = dj b.z + dk b.w (d = neighbour - vertex)
     const double4* tri_k;              // area * (warp, weft, shear), compression ratio
@@ -44,10 +45,6 @@ struct VertexTerms {
 };
 
 constexpr uint32_t kPinnedHead = ~0u;
-// The place of the vertex itself, which its neighbour list leaves out: a hinge can
-// name a vertex twice (two faces on the same three vertices have one vertex as both
-// wings).
-constexpr uint32_t kSelfPlace = (1u << 21) - 1u;
 
 struct SweepView {
     uint32_t n;                 // moving vertices

@@ -448,11 +448,9 @@ struct Near {
         stage(s, r, lane, mask, smem);
         return f;
     }
-    // kSelfPlace: the vertex's position before the solve, as a term's other corners
-    // have it while one corner moves
     __device__ __forceinline__ d3 pos(const SweepView& s, uint32_t i) const {
         if (i < kSlots) return mk(at[i], at[kSlots + i], at[2 * kSlots + i]);
-        return ld3(s.x, i == kSelfPlace ? v : s.vt.nb[nb0 + i]);
+        return ld3(s.x, s.vt.nb[nb0 + i]);
     }
 };
 
