@@ -30,7 +30,7 @@ constexpr int kLanes = 4;       // lanes per vertex of the gradient evaluations
 constexpr int kBlocks = kSumBlocks;
 
 // g_out[3v..3v+2] = dE/dx_v at s.x for moving vertex v (0 where pinned)
-template <int G>
+template <int G, bool FAR>
 __global__ void __launch_bounds__(128) k_nt_gradient(SweepView s, double* g_out) {
     __shared__ double near_s[128 / G * Near<G>::kDoubles];
     uint32_t t = blockIdx.x * 128 + threadIdx.x;
@@ -46,9 +46,9 @@ __global__ void __launch_bounds__(128) k_nt_gradient(SweepView s, double* g_out)
     d3 g = mk(0, 0, 0);
     Sym H;
     sym_zero(H);
-    Near<G> T;
+    Near<G, FAR> T;
     T.head(s, v);
-    const typename Near<G>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
+    const typename Near<G, FAR>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
     local_part<true, G, false>(s, T, f, x, lane, g, H);
     if (G > 1) {
         g.x = group_sum<G>(g.x, mask);
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(128) k_nt_gradient(SweepView s, double* g_out)
 
 // Jacobi diagonal of System::diagonal (src/solver.rs:150-161): inertia +
 // shift + the diagonal of every incident term's Hessian; 1 on fixed dofs.
-template <int G>
+template <int G, bool FAR>
 __global__ void __launch_bounds__(128) k_nt_diagonal(SweepView s, double shift, double* diag) {
     __shared__ double near_s[128 / G * Near<G>::kDoubles];
     const uint32_t lane = threadIdx.x & (G - 1);
@@ -76,9 +76,9 @@ __global__ void __launch_bounds__(128) k_nt_diagonal(SweepView s, double shift, 
             continue;
         }
         d3 x = ld3(s.x, v);
-        Near<G> T;
+        Near<G, FAR> T;
         T.head(s, v);
-        const typename Near<G>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
+        const typename Near<G, FAR>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
         d3 g = mk(0, 0, 0);
         Sym H;
         sym_zero(H);
@@ -267,13 +267,15 @@ class Newton {
         SweepView s = pb_.view;
         s.x = const_cast<double4*>(x);
         unsigned grid = (unsigned)(((uint64_t)s.n * kLanes + 127) / 128);
-        if (grid) k_nt_gradient<kLanes><<<grid, 128, 0, st_>>>(s, out);
+        auto kernel = s.vt.far_tri ? k_nt_gradient<kLanes, true> : k_nt_gradient<kLanes, false>;
+        if (grid) kernel<<<grid, 128, 0, st_>>>(s, out);
         CC_CUDA(cudaGetLastError());
     }
     void diagonal(double shift) {
         SweepView s = pb_.view;
         s.x = w_.x.ptr;
-        k_nt_diagonal<kLanes><<<grid_for(kLanes * (size_t)s.n, 128), 128, 0, st_>>>(s, shift, w_.diag.ptr);
+        auto kernel = s.vt.far_tri ? k_nt_diagonal<kLanes, true> : k_nt_diagonal<kLanes, false>;
+        kernel<<<grid_for(kLanes * (size_t)s.n, 128), 128, 0, st_>>>(s, shift, w_.diag.ptr);
     }
     double read_scalar() {
         CC_CUDA(cudaMemcpyAsync(w_.h_scalar.ptr, w_.scalars.ptr, sizeof(double), cudaMemcpyDeviceToHost, st_));

@@ -472,6 +472,7 @@ struct cc_solver {
     DBuf<uint2> inc_mid;  // per vertex: first hinge entry, first stitch entry
     // per-vertex records of the elastic terms (VertexTerms)
     DBuf<double4> vt_buf;  // one allocation
+    DBuf<uint32_t> vt_far;
     VertexTerms vt{};
     DBuf<uint4> vt_heads;  // in colour order, of the last colouring
     DBuf<uint8_t> pinned;
@@ -1318,7 +1319,7 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
             const cc_material& M = mesh->materials[k];
             mats.push_back({M.warp, M.weft, M.shear, M.compression_ratio, M.compression_transition});
         }
-        if (mats.empty() || mats.size() >> 22) throw Failure{CC_ERR_INVALID_ARGUMENT, "Invalid material binding or mesh topology"};
+        if (mats.empty()) throw Failure{CC_ERR_INVALID_ARGUMENT, "Invalid material binding or mesh topology"};
         auto grain = [&](uint32_t mat, double& sn, double& cs) {
             double r = mesh->materials[mat].grain_degrees * (M_PI / 180.0);
             sn = std::sin(r);
@@ -1397,6 +1398,7 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
         std::vector<uint4> head(2 * n);
         std::vector<uint32_t> nb;
         uint32_t n_vt_tri = 0, n_vt_hinge = 0;
+        bool far = mats.size() > kMaterials;
         for (uint64_t v = 0; v < n; ++v) {
             io[v + 1] = io[v] + (uint32_t)inc[v].size();
             // entries are grouped by type (triangles, hinges, stitches): record the boundaries
@@ -1410,8 +1412,7 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
             const size_t nb0 = nb.size();
             nb.insert(nb.end(), graph[v].begin(), graph[v].end());
             if (twice[v]) nb.insert(std::lower_bound(nb.begin() + nb0, nb.end(), (uint32_t)v), (uint32_t)v);
-            if ((nb.size() - nb0) >> 21)  // the records' 21-bit places
-                throw Failure{CC_ERR_INVALID_ARGUMENT, "a vertex has more than 2^21 mesh neighbours"};
+            far = far || nb.size() - nb0 > kPlaces;
             head[2 * v] = make_uint4((uint32_t)nb0, (uint32_t)(nb.size() - nb0), n_vt_tri, hb - io[v]);
             head[2 * v + 1] = make_uint4(n_vt_hinge, ends, sb - hb - ends, io[v + 1] - sb);
             n_vt_tri += hb - io[v];
@@ -1468,11 +1469,17 @@ int32_t cc_solver_create(const cc_mesh* mesh, const cc_surface* obstacle, const 
             ulonglong2* hinge = reinterpret_cast<ulonglong2*>(tri_k + t);
             unsigned long long* tri = reinterpret_cast<unsigned long long*>(hinge + n_vt_hinge);
             uint32_t* nb_d = reinterpret_cast<uint32_t*>(tri + t);
-            h->vt = {head_d, nb_d, tri, tri_b, tri_k, hinge};
+            uint32_t *far_tri = nullptr, *far_hinge = nullptr;
+            if (far) {
+                h->vt_far.reserve(3 * (t + n_vt_hinge) + 1);
+                far_tri = h->vt_far.ptr;
+                far_hinge = far_tri + 3 * t;
+            }
+            h->vt = {head_d, nb_d, tri, tri_b, tri_k, hinge, far_tri, far_hinge};
             if (n) CC_CUDA(cudaMemcpyAsync(head_d, head.data(), 2 * n * sizeof(uint4), cudaMemcpyHostToDevice, st));
             if (!nb.empty()) CC_CUDA(cudaMemcpyAsync(nb_d, nb.data(), 4 * nb.size(), cudaMemcpyHostToDevice, st));
             launch_vertex_terms(h->sweep_view(h->world->contacts(), cc_vbd_settings{}, nullptr), tri, tri_b, tri_k,
-                                hinge, st);
+                                hinge, far_tri, far_hinge, st);
         }
         h->lo_off.upload(lo_o, st);
         h->lo.upload(lo_v, st);

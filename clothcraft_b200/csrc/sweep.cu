@@ -36,10 +36,10 @@ namespace cc {
 
 // Solves vertex i of the colour; `wait`: the group's first vertex of the launch.
 // False if the launch is to be skipped.
-template <int G>
+template <int G, bool FAR>
 __device__ __forceinline__ bool solve_vertex(const SweepView& s, uint32_t i, uint32_t lane, unsigned mask, double* smem,
                                              bool wait) {
-    Near<G> T;
+    Near<G, FAR> T;
     T.head_of_color(s, i);
     const uint32_t v = T.v;
     const bool pinned = T.nt == kPinnedHead;
@@ -49,8 +49,8 @@ __device__ __forceinline__ bool solve_vertex(const SweepView& s, uint32_t i, uin
     const double m = s.inertia[v];
     const d3 ctr = ld3(s.contacts.centers, v);
     const double rad = s.contacts.radii[v];
-    typename Near<G>::Ids ids = T.ids(s, lane);
-    const typename Near<G>::First f = T.first(s, lane);
+    typename Near<G, FAR>::Ids ids = T.ids(s, lane);
+    const typename Near<G, FAR>::First f = T.first(s, lane);
     if (wait) {
         // up to here only what earlier launches than the last one wrote; now the positions
         wait_for_last_launch();
@@ -131,7 +131,7 @@ __device__ __forceinline__ bool solve_vertex(const SweepView& s, uint32_t i, uin
 // MINB blocks of BLOCK threads per SM caps the registers (65536 / (MINB*BLOCK)).
 // Each group of G lanes solves vertices gi, gi + groups in the grid, ...: one
 // vertex per group when the grid covers the colour, several in a persistent grid.
-template <int G, int BLOCK, int MINB>
+template <int G, int BLOCK, int MINB, bool FAR = false>
 __global__ void __launch_bounds__(BLOCK, MINB) k_sweep(SweepView s, uint32_t count) {
     constexpr uint32_t kGroups = BLOCK / G;
     __shared__ double near_s[kGroups * Near<G>::kDoubles];
@@ -140,18 +140,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_sweep(SweepView s, uint32_t cou
     // whole groups step together; a grid has no more blocks than the colour needs, so a block's first group has a vertex
     bool wait = true;
     for (uint32_t gi = blockIdx.x * kGroups + threadIdx.x / G; gi < count; gi += gridDim.x * kGroups) {
-        if (!solve_vertex<G>(s, gi, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles, wait)) return;
+        if (!solve_vertex<G, FAR>(s, gi, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles, wait)) return;
         wait = false;
     }
     stamp_block_end(s);
 }
 
-template <int G, int B, int MINB>
+template <int G, int B, int MINB, bool FAR = false>
 static void launch_k(const SweepView& s, uint32_t count, cudaStream_t st, unsigned cap) {
     uint64_t threads = (uint64_t)count * G;
     unsigned grid = (unsigned)((threads + B - 1) / B);
     if (cap && grid > cap) grid = cap;
-    launch_after(k_sweep<G, B, MINB>, grid, B, st, s, count);
+    launch_after(k_sweep<G, B, MINB, FAR>, grid, B, st, s, count);
 }
 
 template <int G, int B, int MINB>
@@ -234,6 +234,7 @@ struct SweepResident {
 
 void launch_sweep(const SweepView& s, uint32_t count, int variant, cudaStream_t st, unsigned grid_cap) {
     if (count == 0) return;
+    if (s.vt.far_tri) return launch_k<8, 128, 3, true>(s, count, st, 0u);  // one variant
     SweepVariant v = decode_variant(variant);
     dispatch(v, SweepLaunch{s, count, st, v.persistent ? grid_cap : 0u});
 }
@@ -242,16 +243,16 @@ unsigned sweep_resident_blocks(int variant) { return dispatch(decode_variant(var
 
 // Probe: local e, g, H of every moving vertex at the current positions
 // (the f64 gradient check of src/gpu_vbd.rs:305-379, probe of vbd.wgsl:142-147).
-template <int G>
+template <int G, bool FAR>
 __global__ void __launch_bounds__(128) k_local_blocks(SweepView s, double* energy, double* grad, double* hess) {
     __shared__ double near_s[128 / G * Near<G>::kDoubles];
     const uint32_t lane = threadIdx.x & (G - 1);
     const unsigned mask = ((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1));
     for (uint32_t v = (blockIdx.x * 128 + threadIdx.x) / G; v < s.n; v += gridDim.x * 128 / G) {
         d3 x = ld3(s.x, v);
-        Near<G> T;
+        Near<G, FAR> T;
         T.head(s, v);
-        const typename Near<G>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
+        const typename Near<G, FAR>::First f = T.load(s, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles);
         d3 g = mk(0, 0, 0);
         Sym H;
         sym_zero(H);
@@ -281,7 +282,8 @@ __global__ void __launch_bounds__(128) k_local_blocks(SweepView s, double* energ
 }
 
 void launch_local_blocks(const SweepView& s, double* energy, double* grad, double* hess, cudaStream_t st) {
-    k_local_blocks<8><<<grid_for(8 * (size_t)s.n, 128), 128, 0, st>>>(s, energy, grad, hess);
+    auto kernel = s.vt.far_tri ? k_local_blocks<8, true> : k_local_blocks<8, false>;
+    kernel<<<grid_for(8 * (size_t)s.n, 128), 128, 0, st>>>(s, energy, grad, hess);
 }
 
 // Heads in colour order: what a solve needs of its vertex before it can ask for
@@ -304,7 +306,7 @@ void launch_color_heads(const SweepView& s, const uint32_t* order, uint4* heads,
 
 // Records of VertexTerms from the per-element data, one thread per vertex.
 __global__ void k_vertex_terms(SweepView s, unsigned long long* tri, double4* tri_b, double4* tri_k,
-                               ulonglong2* hinge) {
+                               ulonglong2* hinge, uint32_t* far_tri, uint32_t* far_hinge) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < s.n; v += gridDim.x * blockDim.x) {
         const uint4 a = s.vt.head[2 * (size_t)v], b = s.vt.head[2 * (size_t)v + 1];
         auto place = [&](uint32_t id) {  // in the ascending neighbour list
@@ -315,6 +317,12 @@ __global__ void k_vertex_terms(SweepView s, unsigned long long* tri, double4* tr
                 else hi = mid;
             }
             return (unsigned long long)lo;
+        };
+        auto ids = [](uint32_t* to, size_t record, uint32_t i, uint32_t j, uint32_t k) {
+            if (!to) return;
+            to[3 * record] = i;
+            to[3 * record + 1] = j;
+            to[3 * record + 2] = k;
         };
         const uint32_t* inc = s.inc + s.inc_off[v];
         for (uint32_t i = 0; i < a.w; ++i) {
@@ -327,6 +335,7 @@ __global__ void k_vertex_terms(SweepView s, unsigned long long* tri, double4* tr
             const double w0 = -(c.x + c.y), v0 = -(c.z + c.w);
             const uint32_t j = (uint32_t)(slot == 0 ? tv.y : tv.x), k = (uint32_t)(slot == 2 ? tv.y : tv.z);
             tri[a.z + i] = place(j) | place(k) << 21 | (unsigned long long)(uint32_t)tv.w << 42;
+            ids(far_tri, a.z + i, j, k, (uint32_t)tv.w);
             tri_b[a.z + i] = make_double4(slot == 0 ? c.x : w0, slot == 2 ? c.x : c.y, slot == 0 ? c.z : v0,
                                           slot == 2 ? c.z : c.w);
             tri_k[a.z + i] = make_double4(A * M.warp, A * M.weft, A * M.shear, M.c);
@@ -336,16 +345,18 @@ __global__ void k_vertex_terms(SweepView s, unsigned long long* tri, double4* tr
         for (uint32_t i = 0; i < b.y + b.z; ++i) {
             const uint32_t ent = inc[a.w + i], h = ent & 0x0fffffffu, slot = (ent >> 28) & 3u;
             const uint3 q = hinge_points(s.hinge_v[h], slot);
-            hinge[slot < 2 ? ends++ : wings++] = make_ulonglong2(place(q.x) | place(q.y) << 21 | place(q.z) << 42,
-                                             (unsigned long long)__double_as_longlong(s.hinge_k[h]));
+            const uint32_t at = slot < 2 ? ends++ : wings++;
+            hinge[at] = make_ulonglong2(place(q.x) | place(q.y) << 21 | place(q.z) << 42,
+                                        (unsigned long long)__double_as_longlong(s.hinge_k[h]));
+            ids(far_hinge, at, q.x, q.y, q.z);
         }
     }
 }
 
 void launch_vertex_terms(const SweepView& s, unsigned long long* tri, double4* tri_b, double4* tri_k,
-                         ulonglong2* hinge, cudaStream_t st) {
+                         ulonglong2* hinge, uint32_t* far_tri, uint32_t* far_hinge, cudaStream_t st) {
     if (s.n == 0) return;
-    k_vertex_terms<<<grid_for(s.n, 128), 128, 0, st>>>(s, tri, tri_b, tri_k, hinge);
+    k_vertex_terms<<<grid_for(s.n, 128), 128, 0, st>>>(s, tri, tri_b, tri_k, hinge, far_tri, far_hinge);
     CC_CUDA(cudaGetLastError());
 }
 
@@ -357,7 +368,7 @@ void launch_vertex_terms(const SweepView& s, unsigned long long* tri, double4* t
 // of g: the first-order (KKT) residual of the step's ball-constrained
 // problem (ContactSet::truncate, src/ogc/world.rs:91-100). Skipped when
 // *skip_at <= iteration (that iteration never ran).
-template <int G>
+template <int G, bool FAR = false>
 __global__ void __launch_bounds__(128) k_grad_sq(SweepView s, double* out, const unsigned* skip_at, uint32_t iteration,
                                                  int project) {
     __shared__ double near_s[128 / G * Near<G>::kDoubles];
@@ -366,11 +377,11 @@ __global__ void __launch_bounds__(128) k_grad_sq(SweepView s, double* out, const
     if (v >= s.n) return;  // whole groups leave together
     uint32_t lane = threadIdx.x & (G - 1);
     unsigned mask = G >= 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1)));
-    Near<G> T;
+    Near<G, FAR> T;
     T.head(s, v);
     const bool pinned = s.pinned[v] != 0;
-    const typename Near<G>::Ids ids = T.ids(s, lane);
-    const typename Near<G>::First f = T.first(s, lane);
+    const typename Near<G, FAR>::Ids ids = T.ids(s, lane);
+    const typename Near<G, FAR>::First f = T.first(s, lane);
     wait_for_last_launch();
     if (skip_at && *skip_at <= iteration) return;
     if (pinned) {
@@ -404,6 +415,8 @@ void launch_grad_sq(const SweepView& s, double* out, const unsigned* skip_at, ui
     unsigned grid = (unsigned)(((uint64_t)s.n * (uint64_t)G + 127) / 128);
     if (grid == 0) return;
     int p = project ? 1 : 0;
+    if (s.vt.far_tri)
+        return launch_after(k_grad_sq<8, true>, (unsigned)((8ull * s.n + 127) / 128), 128, st, s, out, skip_at, iteration, p);
     switch (G) {
         case 1: launch_after(k_grad_sq<1>, grid, 128, st, s, out, skip_at, iteration, p); break;
         case 2: launch_after(k_grad_sq<2>, grid, 128, st, s, out, skip_at, iteration, p); break;

@@ -42,7 +42,15 @@ struct VertexTerms {
     const double4* tri_b;              // fibre vectors w = dj b.x + dk b.y, v = dj b.z + dk b.w (d = neighbour - vertex)
     const double4* tri_k;              // area * (warp, weft, shear), compression ratio
     const ulonglong2* hinge;           // neighbours a | b << 21 | c << 42 (hinge_points), bits of K
+    // Where a vertex has more neighbours or the mesh more materials than those
+    // fields hold (kPlaces, kMaterials): the ids themselves, three a record, {j, k,
+    // material} and {a, b, c}; null elsewhere. Kernels of their own read them
+    // (Near's FAR): tests for such places in the others, though never taken, took a
+    // 16-vertex patch's step from 970 to 990-1,008 us.
+    const uint32_t* far_tri;
+    const uint32_t* far_hinge;
 };
+constexpr size_t kPlaces = 1u << 21, kMaterials = 1u << 22;
 
 constexpr uint32_t kPinnedHead = ~0u;
 
@@ -130,10 +138,10 @@ inline SweepVariant decode_variant(int v) {
 // valid variants of the FP64 (fp32 = false) and FP32-assembly sweeps
 bool sweep_variant_valid(int v, bool fp32);
 
-// Fills the records of vt (buffers sized by the heads) from the per-element
-// data of s; once per solver.
+// Fills the records of vt (buffers sized by the heads; the far ones may be null)
+// from the per-element data of s; once per solver.
 void launch_vertex_terms(const SweepView& s, unsigned long long* tri, double4* tri_b, double4* tri_k,
-                         ulonglong2* hinge, cudaStream_t st);
+                         ulonglong2* hinge, uint32_t* far_tri, uint32_t* far_hinge, cudaStream_t st);
 // launch helpers (sweep.cu); grid_cap > 0 limits the grid (persistent variants)
 // (s.heads: the colour's)
 void launch_sweep(const SweepView& s, uint32_t count, int variant, cudaStream_t st, unsigned grid_cap = 0);

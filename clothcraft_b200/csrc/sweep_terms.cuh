@@ -356,7 +356,9 @@ __device__ __forceinline__ double grab_term(const SweepView& s, uint32_t v, d3 p
 // neighbours; further ones are read from global memory). A position is read
 // once, by one lane, and all the terms of the derivative pass and of every
 // line-search trial take it from there.
-template <int G>
+// FAR: the corners' and materials' ids come from far_tri and far_hinge, the
+// positions from global memory.
+template <int G, bool FAR = false>
 struct Near {
     static constexpr uint32_t kSlots = G >= 4 ? 24 : (G == 2 ? 16 : 8);
     static constexpr uint32_t kDoubles = 3 * kSlots;  // per group
@@ -448,7 +450,9 @@ struct Near {
         stage(s, r, lane, mask, smem);
         return f;
     }
-    __device__ __forceinline__ d3 pos(const SweepView& s, uint32_t i) const {
+    // the corner at place i of the list, or of id far[j]
+    __device__ __forceinline__ d3 pos(const SweepView& s, uint32_t i, const uint32_t* far, size_t j) const {
+        if (FAR) return ld3(s.x, far[j]);
         if (i < kSlots) return mk(at[i], at[kSlots + i], at[2 * kSlots + i]);
         return ld3(s.x, s.vt.nb[nb0 + i]);
     }
@@ -457,30 +461,36 @@ struct Near {
 // Partial sum of the incident terms dealt to `lane` of a group of G
 // (VbdSolver::local, src/vbd.rs:196-248), with the vertex at p; f holds the
 // lane's first records.
-template <bool D, int G, bool HS = D>
-__device__ __forceinline__ double local_part(const SweepView& s, const Near<G>& T, typename Near<G>::First f, d3 p,
-                                             uint32_t lane, d3& g, Sym& H) {
+template <bool D, int G, bool HS = D, bool FAR>
+__device__ __forceinline__ double local_part(const SweepView& s, const Near<G, FAR>& T,
+                                             typename Near<G, FAR>::First f, d3 p, uint32_t lane, d3& g, Sym& H) {
     constexpr uint32_t kId = (1u << 21) - 1u;
     double e = 0.0;
     for (uint32_t i = lane; i < T.nt; i += G) {
         const unsigned long long t = f.t;
         const double4 b = f.tb, k = f.tk;
         T.tri(s, i + G, f);
-        e += membrane<D, HS>(s, b, k, (uint32_t)(t >> 42), T.pos(s, (uint32_t)t & kId) - p,
-                             T.pos(s, (uint32_t)(t >> 21) & kId) - p, g, H);
+        const size_t far = 3 * (size_t)(T.t0 + i);
+        e += membrane<D, HS>(s, b, k, FAR ? s.vt.far_tri[far + 2] : (uint32_t)(t >> 42),
+                             T.pos(s, (uint32_t)t & kId, s.vt.far_tri, far) - p,
+                             T.pos(s, (uint32_t)(t >> 21) & kId, s.vt.far_tri, far + 1) - p, g, H);
     }
     // edge ends, then wings: the lanes of a round take the same form
     for (uint32_t i = lane; i < T.ne; i += G) {
         const ulonglong2 h = f.edge;
         if (i + G < T.ne) f.edge = s.vt.hinge[T.h0 + i + G];
-        e += bending_edge<D, HS>(__longlong_as_double((long long)h.y), T.pos(s, (uint32_t)h.x & kId),
-                                 T.pos(s, (uint32_t)(h.x >> 21) & kId), T.pos(s, (uint32_t)(h.x >> 42)), p, g, H);
+        const size_t far = 3 * (size_t)(T.h0 + i);
+        e += bending_edge<D, HS>(__longlong_as_double((long long)h.y), T.pos(s, (uint32_t)h.x & kId, s.vt.far_hinge, far),
+                                 T.pos(s, (uint32_t)(h.x >> 21) & kId, s.vt.far_hinge, far + 1),
+                                 T.pos(s, (uint32_t)(h.x >> 42), s.vt.far_hinge, far + 2), p, g, H);
     }
     for (uint32_t i = lane; i < T.nw; i += G) {
         const ulonglong2 h = f.wing;
         if (i + G < T.nw) f.wing = s.vt.hinge[T.h0 + T.ne + i + G];
-        e += bending_wing<D, HS>(__longlong_as_double((long long)h.y), T.pos(s, (uint32_t)h.x & kId),
-                                 T.pos(s, (uint32_t)(h.x >> 21) & kId), T.pos(s, (uint32_t)(h.x >> 42)), p, g, H);
+        const size_t far = 3 * (size_t)(T.h0 + T.ne + i);
+        e += bending_wing<D, HS>(__longlong_as_double((long long)h.y), T.pos(s, (uint32_t)h.x & kId, s.vt.far_hinge, far),
+                                 T.pos(s, (uint32_t)(h.x >> 21) & kId, s.vt.far_hinge, far + 1),
+                                 T.pos(s, (uint32_t)(h.x >> 42), s.vt.far_hinge, far + 2), p, g, H);
     }
     if (T.ns) {
         const uint32_t b1 = s.inc_off[T.v + 1];
