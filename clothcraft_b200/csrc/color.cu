@@ -24,40 +24,33 @@ __device__ __forceinline__ void mark(unsigned long long& mask, uint32_t c, bool&
 
 // Greedy rule for one vertex: smallest colour not used by a lower-index
 // neighbour (material graph, contact co-vertices, grab). color_of(u) gives a
-// neighbour's current colour.
+// neighbour's current colour. One pass over the neighbours per 64 colours; with one
+// per colour above 63, two colourings of a stack of 48 layers (85 colours) took
+// 2,240 ms instead of 600.
 template <class ColorOf>
 __device__ __forceinline__ uint32_t greedy_color(const ColorView& g, uint32_t v, ColorOf color_of) {
-    unsigned long long mask = 0;
-    bool high = false;
-    for (uint32_t k = g.lo_off[v]; k < g.lo_off[v + 1]; ++k) mark(mask, color_of(g.lo[k]), high);
-    for (uint32_t k = g.contacts.inc_off[v]; k < g.contacts.inc_off[v + 1]; ++k) {
-        uint32_t c = g.contacts.inc[k];
-        uint32_t kind = g.contacts.kind[c];
-        uint4 cv = g.contacts.verts[c];
-        uint32_t ids[4] = {cv.x, cv.y, cv.z, cv.w};
-        uint32_t cnt = kind == 0 ? 2u : (kind == 1 ? 3u : 4u);
-        for (uint32_t j = 0; j < cnt; ++j)
-            if (ids[j] < v) mark(mask, color_of(ids[j]), high);
-    }
-    bool in_grab = g.grab_active && (g.grab_v[0] == v || g.grab_v[1] == v || g.grab_v[2] == v);
-    if (in_grab)
-        for (int j = 0; j < 3; ++j)
-            if (g.grab_v[j] < v) mark(mask, color_of(g.grab_v[j]), high);
-    if (~mask != 0ull) return (uint32_t)__ffsll((long long)~mask) - 1;
-    for (uint32_t col = 64;; ++col) {  // more than 64 colours around v: linear search
-        bool used = false;
-        for (uint32_t k = g.lo_off[v]; k < g.lo_off[v + 1] && !used; ++k) used = color_of(g.lo[k]) == col;
-        for (uint32_t k = g.contacts.inc_off[v]; k < g.contacts.inc_off[v + 1] && !used; ++k) {
+    const bool in_grab = g.grab_active && (g.grab_v[0] == v || g.grab_v[1] == v || g.grab_v[2] == v);
+    for (uint32_t base = 0;; base += 64) {
+        unsigned long long mask = 0;
+        auto used = [&](uint32_t u) {
+            const uint32_t c = color_of(u) - base;
+            if (c < 64) mask |= 1ull << c;
+        };
+        for (uint32_t k = g.lo_off[v]; k < g.lo_off[v + 1]; ++k) used(g.lo[k]);
+        for (uint32_t k = g.contacts.inc_off[v]; k < g.contacts.inc_off[v + 1]; ++k) {
             uint32_t c = g.contacts.inc[k];
             uint32_t kind = g.contacts.kind[c];
             uint4 cv = g.contacts.verts[c];
             uint32_t ids[4] = {cv.x, cv.y, cv.z, cv.w};
             uint32_t cnt = kind == 0 ? 2u : (kind == 1 ? 3u : 4u);
-            for (uint32_t j = 0; j < cnt; ++j) used = used || (ids[j] < v && color_of(ids[j]) == col);
+            for (uint32_t j = 0; j < cnt; ++j)
+                if (ids[j] < v) used(ids[j]);
         }
         if (in_grab)
-            for (int j = 0; j < 3; ++j) used = used || (g.grab_v[j] < v && color_of(g.grab_v[j]) == col);
-        if (!used || col >= kMaxColors - 1) return col;
+            for (int j = 0; j < 3; ++j)
+                if (g.grab_v[j] < v) used(g.grab_v[j]);
+        if (~mask != 0ull) return min(base + (uint32_t)__ffsll((long long)~mask) - 1, (uint32_t)kMaxColors - 1);
+        if (base + 64 >= kMaxColors) return kMaxColors - 1;
     }
 }
 
