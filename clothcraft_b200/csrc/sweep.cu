@@ -36,10 +36,10 @@ namespace cc {
 
 // Solves vertex i of the colour; `wait`: the group's first vertex of the launch.
 // False if the launch is to be skipped.
-template <int G, bool FAR>
+template <int G, bool FAR, bool LEAN>
 __device__ __forceinline__ bool solve_vertex(const SweepView& s, uint32_t i, uint32_t lane, unsigned mask, double* smem,
                                              bool wait) {
-    Near<G, FAR> T;
+    Near<G, FAR, LEAN> T;
     T.head_of_color(s, i);
     const uint32_t v = T.v;
     const bool pinned = T.nt == kPinnedHead;
@@ -49,8 +49,8 @@ __device__ __forceinline__ bool solve_vertex(const SweepView& s, uint32_t i, uin
     const double m = s.inertia[v];
     const d3 ctr = ld3(s.contacts.centers, v);
     const double rad = s.contacts.radii[v];
-    typename Near<G, FAR>::Ids ids = T.ids(s, lane);
-    const typename Near<G, FAR>::First f = T.first(s, lane);
+    typename Near<G, FAR, LEAN>::Ids ids = T.ids(s, lane);
+    const typename Near<G, FAR, LEAN>::First f = T.first(s, lane);
     if (wait) {
         // up to here only what earlier launches than the last one wrote; now the positions
         wait_for_last_launch();
@@ -134,13 +134,22 @@ __device__ __forceinline__ bool solve_vertex(const SweepView& s, uint32_t i, uin
 template <int G, int BLOCK, int MINB, bool FAR = false>
 __global__ void __launch_bounds__(BLOCK, MINB) k_sweep(SweepView s, uint32_t count) {
     constexpr uint32_t kGroups = BLOCK / G;
-    __shared__ double near_s[kGroups * Near<G>::kDoubles];
+    // Few lanes at a budget of 96 registers or fewer (one lane: 128): records and
+    // neighbours loaded as they are needed. Held ahead they spilled ~1,100 bytes a
+    // thread at 80 registers and ~2,000 at 64, with half the L1 taken by the staged
+    // positions: a 640 x 640 crumple's sweeps of a step at 1, 2 and 4 lanes and 64
+    // registers took 78, 51 and 39 ms, 54, 36 and 29 now; at 168 registers (23 ms at
+    // 4 lanes) loading ahead is the better form. From 8 lanes on the compiler
+    // contracts the two forms differently, and a cap must not change a step's bits.
+    constexpr bool kLean = G <= 4 && MINB * BLOCK > (G == 1 ? 3 : 4) * 128;
+    constexpr uint32_t kDoubles = Near<G, FAR, kLean>::kDoubles;
+    __shared__ double near_s[kGroups * kDoubles];
     const uint32_t lane = threadIdx.x & (G - 1);
     const unsigned mask = G >= 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(unsigned)(G - 1)));
     // whole groups step together; a grid has no more blocks than the colour needs, so a block's first group has a vertex
     bool wait = true;
     for (uint32_t gi = blockIdx.x * kGroups + threadIdx.x / G; gi < count; gi += gridDim.x * kGroups) {
-        if (!solve_vertex<G, FAR>(s, gi, lane, mask, near_s + threadIdx.x / G * Near<G>::kDoubles, wait)) return;
+        if (!solve_vertex<G, FAR, kLean>(s, gi, lane, mask, near_s + threadIdx.x / G * kDoubles, wait)) return;
         wait = false;
     }
     stamp_block_end(s);

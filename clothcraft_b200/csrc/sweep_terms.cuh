@@ -357,10 +357,10 @@ __device__ __forceinline__ double grab_term(const SweepView& s, uint32_t v, d3 p
 // once, by one lane, and all the terms of the derivative pass and of every
 // line-search trial take it from there.
 // FAR: the corners' and materials' ids come from far_tri and far_hinge, the
-// positions from global memory.
-template <int G, bool FAR = false>
+// positions from global memory. LEAN: nothing is loaded ahead (few registers).
+template <int G, bool FAR = false, bool LEAN = false>
 struct Near {
-    static constexpr uint32_t kSlots = G >= 4 ? 24 : (G == 2 ? 16 : 8);
+    static constexpr uint32_t kSlots = G >= 4 ? 24 : (LEAN ? 4 * G : 8 * G);
     static constexpr uint32_t kDoubles = 3 * kSlots;  // per group
     uint32_t v, nb0, n_nb, t0, nt, h0, ne, nw, ns, c0, c1;
     double* at;  // x, y and z of the staged positions
@@ -406,6 +406,7 @@ struct Near {
     }
     __device__ __forceinline__ First first(const SweepView& s, uint32_t lane) const {
         First f{};
+        if (LEAN) return f;
         tri(s, lane, f);
         if (lane < ne) f.edge = s.vt.hinge[h0 + lane];
         if (lane < nw) f.wing = s.vt.hinge[h0 + ne + lane];
@@ -419,7 +420,8 @@ struct Near {
         uint32_t id[kPer];
     };
     __device__ __forceinline__ Ids ids(const SweepView& s, uint32_t lane) const {
-        Ids r;
+        Ids r{};
+        if (LEAN) return r;
         const uint32_t m = min(n_nb, kSlots);
 #pragma unroll
         for (int j = 0; j < kPer; ++j) r.id[j] = lane + j * G < m ? s.vt.nb[nb0 + lane + j * G] : 0u;
@@ -428,6 +430,18 @@ struct Near {
     __device__ __forceinline__ void stage(const SweepView& s, const Ids& r, uint32_t lane, unsigned mask, double* smem) {
         at = smem;
         const uint32_t m = min(n_nb, kSlots);
+        if (LEAN) {
+            __syncwarp(mask);
+#pragma unroll 1
+            for (uint32_t k = lane; k < m; k += G) {
+                const d3 q = ld3(s.x, s.vt.nb[nb0 + k]);
+                at[k] = q.x;
+                at[kSlots + k] = q.y;
+                at[2 * kSlots + k] = q.z;
+            }
+            __syncwarp(mask);
+            return;
+        }
         d3 q[kPer];
 #pragma unroll
         for (int j = 0; j < kPer; ++j)
@@ -461,15 +475,17 @@ struct Near {
 // Partial sum of the incident terms dealt to `lane` of a group of G
 // (VbdSolver::local, src/vbd.rs:196-248), with the vertex at p; f holds the
 // lane's first records.
-template <bool D, int G, bool HS = D, bool FAR>
-__device__ __forceinline__ double local_part(const SweepView& s, const Near<G, FAR>& T,
-                                             typename Near<G, FAR>::First f, d3 p, uint32_t lane, d3& g, Sym& H) {
+template <bool D, int G, bool HS = D, bool FAR, bool LEAN>
+__device__ __forceinline__ double local_part(const SweepView& s, const Near<G, FAR, LEAN>& T,
+                                             typename Near<G, FAR, LEAN>::First f, d3 p, uint32_t lane, d3& g,
+                                             Sym& H) {
     constexpr uint32_t kId = (1u << 21) - 1u;
     double e = 0.0;
     for (uint32_t i = lane; i < T.nt; i += G) {
+        if (LEAN) T.tri(s, i, f);
         const unsigned long long t = f.t;
         const double4 b = f.tb, k = f.tk;
-        T.tri(s, i + G, f);
+        if (!LEAN) T.tri(s, i + G, f);
         const size_t far = 3 * (size_t)(T.t0 + i);
         e += membrane<D, HS>(s, b, k, FAR ? s.vt.far_tri[far + 2] : (uint32_t)(t >> 42),
                              T.pos(s, (uint32_t)t & kId, s.vt.far_tri, far) - p,
@@ -477,16 +493,16 @@ __device__ __forceinline__ double local_part(const SweepView& s, const Near<G, F
     }
     // edge ends, then wings: the lanes of a round take the same form
     for (uint32_t i = lane; i < T.ne; i += G) {
-        const ulonglong2 h = f.edge;
-        if (i + G < T.ne) f.edge = s.vt.hinge[T.h0 + i + G];
+        const ulonglong2 h = LEAN ? s.vt.hinge[T.h0 + i] : f.edge;
+        if (!LEAN && i + G < T.ne) f.edge = s.vt.hinge[T.h0 + i + G];
         const size_t far = 3 * (size_t)(T.h0 + i);
         e += bending_edge<D, HS>(__longlong_as_double((long long)h.y), T.pos(s, (uint32_t)h.x & kId, s.vt.far_hinge, far),
                                  T.pos(s, (uint32_t)(h.x >> 21) & kId, s.vt.far_hinge, far + 1),
                                  T.pos(s, (uint32_t)(h.x >> 42), s.vt.far_hinge, far + 2), p, g, H);
     }
     for (uint32_t i = lane; i < T.nw; i += G) {
-        const ulonglong2 h = f.wing;
-        if (i + G < T.nw) f.wing = s.vt.hinge[T.h0 + T.ne + i + G];
+        const ulonglong2 h = LEAN ? s.vt.hinge[T.h0 + T.ne + i] : f.wing;
+        if (!LEAN && i + G < T.nw) f.wing = s.vt.hinge[T.h0 + T.ne + i + G];
         const size_t far = 3 * (size_t)(T.h0 + T.ne + i);
         e += bending_wing<D, HS>(__longlong_as_double((long long)h.y), T.pos(s, (uint32_t)h.x & kId, s.vt.far_hinge, far),
                                  T.pos(s, (uint32_t)(h.x >> 21) & kId, s.vt.far_hinge, far + 1),
@@ -498,9 +514,10 @@ __device__ __forceinline__ double local_part(const SweepView& s, const Near<G, F
             e += stitch_term<D>(s, s.inc[k] & 0x0fffffffu, T.v, p, g, H);
     }
     for (uint32_t k = T.c0 + lane; k < T.c1; k += G) {
+        if (LEAN) T.contact(s, k, f);
         const uint4 c = f.c;
         const double eps = f.eps;
-        T.contact(s, k + G, f);
+        if (!LEAN) T.contact(s, k + G, f);
         e += contact_rec<D, HS>(s, c, eps, p, g, H);
     }
     if (lane == 0 && s.grab.active && (s.grab.v[0] == T.v || s.grab.v[1] == T.v || s.grab.v[2] == T.v))
