@@ -179,7 +179,12 @@ __device__ __forceinline__ void wait_for_last_launch() {
 
 // Launches a kernel that may start while the launch before it in the stream
 // drains (programmatic dependent launch); the kernel waits for that launch
-// itself (wait_for_last_launch) before it reads what it wrote. A chain of short
+// itself (wait_for_last_launch) before it reads what that one wrote. What a kernel
+// reads before its wait must not be written by a kernel directly ahead of it: the
+// sweeps and the residual gradient read heads, records, neighbour ids and pinned
+// flags there, the sweeps targets, inertia and balls as well, all of which detection
+// and colouring write, with k_batch_begin (an ordinary launch) or a copy between
+// them and the first sweep. A chain of short
 // launches is bound by each one's start and first loads: the sweeps of a 16-vertex
 // patch went 0.630 -> 0.563 ms a step (96 launches), of the fold 7.27 -> 7.08.
 template <class... P, class... A>

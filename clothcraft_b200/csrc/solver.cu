@@ -773,7 +773,8 @@ struct cc_solver {
 // a backup of the positions (restored after each trial) and keep the fastest.
 void cc_solver::autotune(const SweepView& sv_in, bool fp32) {
     // lanes per vertex | register cap (resident 128-thread blocks per SM: 3, 4, 5,
-    // 6 or 8; above 3 the compiler spills to local memory) << 8
+    // 6 or 8; the FP64 sweep spills to local memory above 3, with 1 to 4 lanes ~100
+    // bytes at 3 as well) << 8
     // | kVariantPersistent: a grid of the resident blocks looping over the colour;
     // | 1 << 17 or 2 << 17: blocks of 64 or 256 threads at the same register budget
     constexpr int P = kVariantPersistent, B64 = 1 << 17, B256 = 2 << 17;
@@ -940,12 +941,11 @@ void cc_solver::step(const cc_vbd_settings& s, const cc_grab* grab, cc_metrics* 
     CC_CUDA(cudaGetLastError());
     read_scalars();
     size_t clipped = sc_h.ptr->clipped;
-    // Iterations are enqueued ahead of the device: k_refresh_rule (and, with a
-    // residual target, k_residual_rule) decide on the device and later sweeps
-    // exit at once. Without a target all iterations go in one batch and the
-    // host syncs once; with one, they go in chunks and the host reads the
-    // previous chunk's stop flag while the next chunk runs. After a refresh
-    // the host redoes detection and colouring and resumes at that iteration.
+    // Iterations are enqueued ahead of the device in chunks (below): k_refresh_rule
+    // (and, with a residual target, k_residual_rule) decide on the device, and
+    // sweeps enqueued past a stop exit at once. With or without a target the host
+    // reads a chunk's stop word while the next chunk runs. After a refresh it
+    // redoes detection and colouring and resumes at that iteration.
     const double threshold = s.contact.refresh_fraction * (double)n;
     const double tol2 = s.residual_tolerance * s.residual_tolerance;
     const bool target_on = s.residual_tolerance > 0.0;

@@ -27,8 +27,9 @@
 // (solve_vertex), the records (VertexTerms), the positions staged once (Near) and
 // the launches that start while the last one drains (launch_after). A launch on
 // the fold (16k vertices, 8 lanes, cold caches): 39.9 us with per-element data and
-// generic second derivatives (spilling at 128 registers), 26.6 us now (168, none); a 640 x 640 crumple's sweeps of a step
-// (410k vertices, 40 iterations) 31.1 -> 21.5 ms. With the records in their loops
+// generic second derivatives (128 registers, with spills), 26.7 us now (168, none; at
+// 168, spills of 56 to 104 bytes only with 1 to 4 lanes); a 640 x 640 crumple's
+// sweeps of a step (410k vertices, 40 iterations) 31.1 -> 21.5 ms. With the records in their loops
 // instead of loaded ahead, the crumple took 27.2 ms.
 #include "sweep_terms.cuh"
 

@@ -54,6 +54,9 @@ constexpr size_t kPlaces = 1u << 21, kMaterials = 1u << 22;
 
 constexpr uint32_t kPinnedHead = ~0u;
 
+// k_sweep and k_grad_sq may read everything here but x, residual, the counters and skip_at
+// before they wait for the launch ahead of them (launch_after): no kernel launched
+// directly ahead of one of them writes it.
 struct SweepView {
     uint32_t n;                 // moving vertices
     double4* x;                 // [n_all] positions (moving part written)

@@ -245,13 +245,17 @@ class World {
     DBuf<double4> centers_;
     DBuf<uint32_t> inc_count_, inc_off_, inc_cursor_;
     // per incidence: the record as the row's vertex sees it, its epsilon, the
-    // contact id, and the id as the rows were dealt; one allocation
+    // contact id, and the id as the rows were dealt; one allocation, for four moving
+    // vertices of every contact before the duplicates go (128 bytes each), since the
+    // host learns the contacts' number with the detection's last read-back
     DBuf<uint4> inc_buf_;
     uint4* inc_ref_ = nullptr;
     double* inc_eps_ = nullptr;
     uint32_t *inc_ = nullptr, *inc_raw_ = nullptr;
     RadixSorter sorter_;
-    DBuf<uint8_t> fetch_d_;    // kinds, counts and 64-bit offsets of fetch()
+    // kinds, counts and 64-bit offsets of fetch(), and its pinned copy of the whole set: kept with the world, at 1.5
+    // times the largest set fetched
+    DBuf<uint8_t> fetch_d_;
     Pinned<uint8_t> fetch_h_;
     DBuf<uint32_t> scan_tmp_;
     DBuf<DetectStats> stats_d_;

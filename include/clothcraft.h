@@ -316,8 +316,8 @@ int32_t cc_solver_set_graphs(cc_solver* solver, int32_t enable);
 int32_t cc_solver_set_profiling(cc_solver* solver, int32_t enable);
 /* Threads that cooperate on one vertex's local solve (1, 2, 4, 8, 16 or 32),
  * optionally | (cap << 8) with cap = 3, 4, 5, 6 or 8 resident 128-thread
- * blocks per SM (a register budget; default 3; above 3 registers spill to
- * local memory), | (1 << 16) for a persistent grid (at most the resident
+ * blocks per SM (a register budget; default 3; above 3, and with 1 to 4
+ * lanes at 3, registers spill to local memory), | (1 << 16) for a persistent grid (at most the resident
  * blocks, each looping over the colour's vertices), | (1 << 17) or (2 << 17)
  * for blocks of 64 or 256 threads (4 or 8 lanes; caps 3-4 or 4, 6, 8) at the
  * same register budget; 0 (the default) lets the solver time the
