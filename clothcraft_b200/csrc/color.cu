@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(128) k_color_rows(ColorView g, ColorRows r, co
 // sheet, a roll), and the lookup of changed vertices' neighbours and the rows
 // loaded on demand (~2 us a chunk) would save nothing. On the 40k-vertex garment,
 // whose contacts change by a few between refreshes, it leaves out 40 % of the
-// chunks: 0.22 -> 0.18 ms a colouring.
+// chunks: 0.22 -> 0.17 ms a colouring (host clock, with its sort and heads).
 //
 // What bounds it: the chain of chunks, each a row load, a gather of final
 // colours and two to three barrier rounds; the next chunk's row is loaded
