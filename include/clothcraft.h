@@ -323,7 +323,8 @@ int32_t cc_solver_set_profiling(cc_solver* solver, int32_t enable);
  * same register budget; 0 (the default) lets the solver time the
  * candidates on its first step and keep the fastest. get_lanes returns the
  * same encoding. Two solvers take bitwise-identical steps only with the same
- * setting. No reference counterpart (the wgpu backend always uses a 32-lane
+ * setting. A mesh of more than 2^22 materials, or with more than 2^21 mesh
+ * neighbours of one vertex, has one variant whatever is set. No reference counterpart (the wgpu backend always uses a 32-lane
  * workgroup per vertex, src/vbd.wgsl:118-150). */
 int32_t cc_solver_set_lanes(cc_solver* solver, int32_t lanes);
 int32_t cc_solver_get_lanes(const cc_solver* solver);
